@@ -345,18 +345,18 @@ typedef struct {
     float du, dv, su, sv, d_pix, DSO, DSD;
 } vg_dd3d_geom;
 
-/* Device workspace (per-view line scales and z magnifications) both cone
- * calls need; 0 for an invalid geometry. */
+/* Device workspace (per-view line scales and z magnifications, 16-byte
+ * aligned) both cone calls need; 0 for an invalid geometry. */
 size_t vg_dd3d_workspace_bytes(const vg_dd3d_geom *g);
 
 /* Forward projection (dd.py:815-825, sweep :285-380 as intended; returns
- * sino * d_pix^2 / (du dv)), one thread per (view, u, v) bin. */
+ * sino * d_pix^2 / (du dv)); a warp per 8 u cells of a view. */
 int vg_dd3d_fp(const vg_dd3d_geom *g, const float *vol, const double *trig,
                float *sino, void *workspace, size_t workspace_bytes,
                void *stream);
 
 /* Backprojection (dd.py:829-835, sweep :384-468; returns img / (na d_pix)),
- * one thread per voxel. */
+ * a warp per 8 voxel columns. */
 int vg_dd3d_bp(const vg_dd3d_geom *g, const float *sino, const double *trig,
                float *vol, void *workspace, size_t workspace_bytes,
                void *stream);
