@@ -178,13 +178,13 @@ typedef struct {
                         0 = chosen from the sizes (vg_dd2d_fp_default_variant) */
 } vg_dd2d_geom;
 
-/* Number of forward-projector tile variants, and the one variant 0 maps to
- * for a geometry (the autotuner in vir_gb300/autotune.py times the others). */
+/* Number of forward-projector variants (the last: the fan beam's tap form; a
+ * geometry it does not serve falls back to the tile chosen by size), and the
+ * one variant 0 maps to for a geometry (vir_gb300/autotune.py times the others). */
 int vg_dd2d_fp_variants(void);
 int vg_dd2d_fp_default_variant(const vg_dd2d_geom *g);
 
-/* Forward projection, gather form (one thread per bin, pixels of each
- * orthogonal line found directly), returns A x * d_pix / du exactly as
+/* Forward projection, gather form, returns A x * d_pix / du exactly as
  * dd_fp_par_2d / dd_fp_fan_2d (dd.py:651-661, 725; 730-736, 803).
  * img is (nx, ny); imgT is its transpose (ny, nx) (the caller keeps both so
  * that both driving axes read contiguous lines); sino (na, nu). */

@@ -1,0 +1,78 @@
+"""The fan-beam forward projection's tap form (vg_dd2d_fp_variants' last
+variant) and the back projection's view split, where they change form: bins
+of up to 1, 2, 3 and more pixels, odd and one-line images, few views (bins of
+a view over several blocks, lines over several warps), a detector near its
+inverse map's pole (the exact share), whole views of more than 768 bins in the
+SIRT epilogue, 1, 2 and 4 blocks of views per tile.
+
+Tolerance: bin positions carry three float32 roundings of at most two image
+widths, 7e-5 pixel for the sizes here, on pixel steps of at most 1: 1e-4 of the
+largest value against the FP64 oracle, as for the integral form."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# shape, nu, na, du, su, d_pix, DSO, DSD
+CASES = {
+    "fine": ((65, 64), 190, 7, 0.4, 0.0, 1.0, 90.0, 170.0),      # bins of 0.2-0.5 pixel
+    "mid": ((48, 53), 61, 33, 1.6, 0.25, 1.0, 60.0, 100.0),      # about 1; odd lines
+    "wide": ((40, 40), 32, 70, 2.2, -0.5, 1.0, 34.0, 52.0),      # up to 3 and more near the edges
+    "line": ((1, 37), 40, 130, 1.0, 0.0, 1.0, 60.0, 80.0),       # a single line or pixel row
+    "pole": ((24, 24), 330, 9, 0.7, 0.0, 1.0, 90.0, 130.0),      # detector out to 0.89 DSD
+    "tall": ((200, 9), 260, 3, 1.0, 0.0, 1.0, 220.0, 300.0),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_taps_vs_oracle(vg, orc, name):
+    from vir_gb300 import _lib
+    from vir_gb300.sys_mat import dd
+    shape, nu, na, du, su, d, DSO, DSD = CASES[name]
+    g = _lib.DD2DGeom(*shape, na, nu, du, su, d, DSO, DSD, 1)
+    L = _lib.load()
+    assert L.vg_dd2d_fp_default_variant(ctypes.byref(g)) == L.vg_dd2d_fp_variants()
+    rng = np.random.default_rng(29)
+    img = rng.random(shape).astype(np.float32)
+    y = rng.random((na, nu)).astype(np.float32)
+    angs = np.linspace(0, 2 * np.pi, na, endpoint=False) + 0.02
+    kw = dict(du=du, su=su, d_pix=d)
+    for got, ref in ((dd.dd_fp_fan_2d(img, angs, nu, DSO, DSD, **kw),
+                      orc.dd_fp_fan_2d(img, angs, nu, DSO, DSD, **kw)),
+                     (dd.dd_bp_fan_2d(y, angs, shape, DSO, DSD, **kw),
+                      orc.dd_bp_fan_2d(y, angs, shape, DSO, DSD, **kw))):
+        assert np.abs(got - ref).max() <= 1e-4 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("nu", [96, 801])
+def test_taps_sirt_epilogue_vs_oracle(vg, orc, nu):
+    """Three SIRT updates: the residual and its back projection tables from the
+    tap form's epilogue, with one block per view (2e-4 as the other SIRT tests)."""
+    from vir_gb300 import reconstruction as rc
+    rng = np.random.default_rng(31)
+    shape, na, DSO, DSD = (45, 50), 66, 70.0, 120.0
+    du = 110.0 / nu
+    img = rng.random(shape).astype(np.float32)
+    angs = np.linspace(0, 2 * np.pi, na, endpoint=False)
+    fp = lambda x: orc.dd_fp_fan_2d(x, angs, nu, DSO, DSD, du=float(np.float32(du)))
+    bp = lambda s: orc.dd_bp_fan_2d(s, angs, shape, DSO, DSD, du=float(np.float32(du)))
+    y = fp(img).astype(np.float32)
+    xo = orc.sirt(y, fp, bp, shape, iters=4)
+    x = rc.sirt_2d(y, angs, shape, geom="fan", DSO=DSO, DSD=DSD, du=du, iters=4)
+    assert np.abs(x - xo).max() <= 2e-4 * np.abs(xo).max()
+
+
+def test_taps_nan_stays_near(vg):
+    """A NaN pixel reaches only the bins within two of those it projects to."""
+    import torch
+    from vir_gb300.sys_mat import dd
+    angs = np.linspace(0.1, 6.0, 8)
+    x = torch.rand((40, 44), generator=torch.Generator().manual_seed(1)).cuda()
+    hit = torch.zeros_like(x)
+    hit[17, 21] = 1.0
+    fp = lambda t: dd.dd_fp_fan_2d(t, angs, 90, 60.0, 100.0, du=1.0)
+    near = torch.nn.functional.max_pool1d((fp(hit) != 0).float()[:, None], 5, 1, 2)[:, 0] > 0
+    x[17, 21] = float("nan")
+    assert not bool((torch.isnan(fp(x)) & ~near).any())
