@@ -37,6 +37,7 @@
 // coefficient is negative the edge order is reversed, as dd.py:516-518 does.
 #include "vg_common.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -61,6 +62,7 @@
 namespace {
 
 using namespace vg;
+namespace cg = cooperative_groups;
 
 // Storage types of the image (TX) and the measured sinogram (TY): float, or
 // bfloat16 with all arithmetic in float32 (the batched SIRT's bf16 storage).
@@ -872,7 +874,10 @@ dd2d_fp_taps_kernel(vg_dd2d_geom g, const float *__restrict__ img, const float *
 // threads numbered along y first, so that a warp covers 8 x 4 patches
 // (16 x 8 pixels) when BP_TY = 8: its table gathers span fewer bins than a
 // warp along a 64 x 2 strip (0.213 against 0.233 ms at the fan SIRT size,
-// with the view loop unrolled by 4).
+// with the view loop unrolled by 4).  The tiles of a 512 x 512 image are 256
+// blocks, 1.7 per SM: in fan beam a cluster of blocks splits a tile's views until
+// an SM has four, which 64 registers and an unroll of 2 let it hold (0.204 ->
+// 0.184 ms; at 128 registers and an unroll of 4 a split tile takes 0.27 ms).
 #ifndef VG_BP_TY
 #define VG_BP_TY 8
 #endif
@@ -886,6 +891,7 @@ dd2d_fp_taps_kernel(vg_dd2d_geom g, const float *__restrict__ img, const float *
 #define VG_BP_UNROLL 4
 #endif
 constexpr int BP_UNROLL = VG_BP_UNROLL;  // views per unrolled step of the view loop
+constexpr int BP_FILL = 4;  // blocks per SM that the view split aims at
 constexpr int BP_TY = VG_BP_TY;  // patches along y (threadIdx.x, contiguous in img)
 constexpr int BP_TX = VG_BP_TX;  // patches along x (threadIdx.y)
 constexpr int BP_VC = (BP_TY * BP_TX < 128) ? BP_TY * BP_TX : 128;  // views staged per chunk
@@ -936,7 +942,9 @@ __device__ __forceinline__ float fma_sat(float a, float b, float c) {
 // mode 0: img = BP;  mode 1 (SIRT update): x += gamma * BP * inv_w (BP where
 // inv_w == 0), written to x and its transpose xT.
 // One block's work: the pixel tile (tile_y, tile_x) of BP_TY x BP_TX patches.
-template <bool FAN, typename TX, bool COH = false>
+// SPLIT: the tile is shared by the blocks of a cluster, each with a part of the
+// views; their sums are added in rank order through distributed shared memory.
+template <bool FAN, typename TX, bool COH = false, bool SPLIT = false>
 __device__ __forceinline__ void bp_block(const vg_dd2d_geom &g, int tile_y, int tile_x, BpWork w,
                                          const double *__restrict__ trig, TX *__restrict__ img,
                                          int mode, const float *__restrict__ inv_w, float gamma,
@@ -962,8 +970,11 @@ __device__ __forceinline__ void bp_block(const vg_dd2d_geom &g, int tile_y, int 
     const float cx0 = bx + 0.5f * g.d_pix, cy0 = by + 0.5f * g.d_pix;
     const float2 *ts_all = w.ts;
     Kahan acc[2][2];
-    for (int a0 = 0; a0 < g.na; a0 += BP_VC) {
-        const int nv = min(BP_VC, g.na - a0);
+    const int S = SPLIT ? (int)cg::this_cluster().num_blocks() : 1;
+    const int rank = SPLIT ? (int)cg::this_cluster().block_rank() : 0;
+    const int a_end = (int)((long long)g.na * (rank + 1) / S);
+    for (int a0 = (int)((long long)g.na * rank / S); a0 < a_end; a0 += BP_VC) {
+        const int nv = min(BP_VC, a_end - a0);
         __syncthreads();
         if (tid < nv) {
             const ViewGeo v = view_geo(trig, a0 + tid);
@@ -975,7 +986,7 @@ __device__ __forceinline__ void bp_block(const vg_dd2d_geom &g, int tile_y, int 
         __syncthreads();
         if (!inside) continue;
         float part[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll BP_UNROLL
+#pragma unroll(SPLIT ? 2 : BP_UNROLL)
         for (int vi = 0; vi < nv; ++vi) {
             const float4 q = Vs[vi];
             const bool xd = Xs[vi];
@@ -1015,14 +1026,29 @@ __device__ __forceinline__ void bp_block(const vg_dd2d_geom &g, int tile_y, int 
 #pragma unroll
             for (int dy = 0; dy < 2; ++dy) acc[dx][dy].add(part[dx][dy]);
     }
-    if (!inside) return;
     const float f = 1.0f / ((float)g.na * g.d_pix);
+    __shared__ float2 sums[SPLIT ? 4 : 1][SPLIT ? BP_TY * BP_TX : 1];  // (sum, compensation)
+    if (SPLIT) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sums[i][tid] = make_float2(acc[i >> 1][i & 1].s, acc[i >> 1][i & 1].c);
+        cg::this_cluster().sync();
+    }
 #pragma unroll
     for (int dx = 0; dx < 2; ++dx)
 #pragma unroll
         for (int dy = 0; dy < 2; ++dy) {
             const int px = ix + dx, py = iy + dy;
             if (px >= g.nx || py >= g.ny) continue;
+            if (SPLIT) {  // each pixel of the patch by one block
+                if ((2 * dx + dy) % S != rank) continue;
+                Kahan a;
+                for (int r = 0; r < S; ++r) {
+                    const float2 q = *cg::this_cluster().map_shared_rank(&sums[2 * dx + dy][tid], r);
+                    a.add(q.x);
+                    a.add(-q.y);
+                }
+                acc[dx][dy] = a;
+            }
             const float bp = acc[dx][dy].s * f;
             const size_t o = (size_t)px * g.ny + py;
             if (mode == 1) {
@@ -1035,14 +1061,39 @@ __device__ __forceinline__ void bp_block(const vg_dd2d_geom &g, int tile_y, int 
                 stf(img + o, bp);
             }
         }
+    if (SPLIT) cg::this_cluster().sync();  // no block leaves while its sums are read
 }
 
-template <bool FAN>
-__global__ void __launch_bounds__(BP_TY * BP_TX, VG_BP_MINB)
+template <bool FAN, bool SPLIT>
+__global__ void __launch_bounds__(BP_TY * BP_TX, SPLIT ? BP_FILL : VG_BP_MINB)
 dd2d_bp_kernel(vg_dd2d_geom g, BpWork w, const double *__restrict__ trig,
                float *__restrict__ img, int mode, const float *__restrict__ inv_w, float gamma,
                float *__restrict__ xT) {
-    bp_block<FAN, float>(g, blockIdx.x, blockIdx.y, w, trig, img, mode, inv_w, gamma, xT);
+    const int S = SPLIT ? (int)cg::this_cluster().num_blocks() : 1;
+    bp_block<FAN, float, false, SPLIT>(g, blockIdx.x / S, blockIdx.y, w, trig, img, mode, inv_w, gamma, xT);
+}
+
+template <bool FAN>
+int launch_bp_t(const vg_dd2d_geom *g, BpWork w, const double *trig, float *img, int mode, const float *inv_w,
+                float gamma, float *xT, cudaStream_t st) {
+    const int ty = ceil_div(g->ny, 2 * BP_TY), tx = ceil_div(g->nx, 2 * BP_TX);
+    VG_REQUIRE(tx < 65536, "dd2d_bp: nx too large");
+    // Fan beam: a cluster per tile until every SM has BP_FILL blocks, 16 views per
+    // block at least.  Parallel sums keep their order: SIRT divides by overlaps that
+    // rounding alone makes at 0 and 90 degrees, and shows a last-bit change as 1e-3.
+    int S = 1;
+    while (FAN && S < 4 && (long long)tx * ty * S < BP_FILL * 152 && g->na >= 32 * S) S *= 2;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(ty * S, tx);
+    c.blockDim = dim3(BP_TY, BP_TX);
+    c.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = S > 1 ? 1 : 0;
+    auto kern = S > 1 ? dd2d_bp_kernel<FAN, true> : dd2d_bp_kernel<FAN, false>;
+    return cuda_status(cudaLaunchKernelEx(&c, kern, *g, w, trig, img, mode, inv_w, gamma, xT), "dd2d_bp");
 }
 
 int check_geom(const vg_dd2d_geom *g) {
@@ -1206,14 +1257,8 @@ int launch_bp(const vg_dd2d_geom *g, const float *sino, const double *trig, floa
         int s = launch_status("dd2d_bp_prep");
         if (s) return s;
     }
-    dim3 grid(ceil_div(g->ny, 2 * BP_TY), ceil_div(g->nx, 2 * BP_TX));
-    VG_REQUIRE(grid.y < 65536, "dd2d_bp: nx too large");
-    dim3 block(BP_TY, BP_TX);
-    if (g->fan)
-        dd2d_bp_kernel<true><<<grid, block, 0, st>>>(*g, w, trig, img, mode, inv_w, gamma, xT);
-    else
-        dd2d_bp_kernel<false><<<grid, block, 0, st>>>(*g, w, trig, img, mode, inv_w, gamma, xT);
-    return launch_status("dd2d_bp");
+    return g->fan ? launch_bp_t<true>(g, w, trig, img, mode, inv_w, gamma, xT, st)
+                  : launch_bp_t<false>(g, w, trig, img, mode, inv_w, gamma, xT, st);
 }
 
 }  // namespace
