@@ -593,43 +593,12 @@ struct TapBin {
     float eps;
 };
 
-// 1 / d to about half an ulp: the hardware's estimate and one Newton step.
-__device__ __forceinline__ float recip_n(float d) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    return fmaf(fmaf(-d, r, 1.0f), r, r);
-}
-
 // Share of a bin before tau (saturated to [0, 1]).
 __device__ __forceinline__ float tap_share(float tau, float eps, float e1) {  // e1 = 1 - eps
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(eps, tau, e1)));
     return __saturatef(tau * r);
 }
-
-// Packed float32 pairs (one instruction each on sm_100 and later).
-__device__ __forceinline__ unsigned long long &u64(float2 &a) { return reinterpret_cast<unsigned long long &>(a); }
-__device__ __forceinline__ float2 pk_fma(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(u64(d)) : "l"(u64(a)), "l"(u64(b)), "l"(u64(c)));
-    return d;
-}
-__device__ __forceinline__ float2 pk_mul(float2 a, float2 b) {
-    float2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(u64(d)) : "l"(u64(a)), "l"(u64(b)));
-    return d;
-}
-__device__ __forceinline__ float2 pk_add(float2 a, float2 b) {
-    float2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(u64(d)) : "l"(u64(a)), "l"(u64(b)));
-    return d;
-}
-__device__ __forceinline__ float2 pk_add_rd(float2 a, float2 b) {
-    float2 d;
-    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(u64(d)) : "l"(u64(a)), "l"(u64(b)));
-    return d;
-}
-__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
 
 // Line pair p of the table: (scale of line 2p, of 2p + 1, 1 / |DSO pd + sigma c| of
 // both), scales times d_pix.

@@ -203,33 +203,6 @@ struct WarpBuf {
     float4 line[4];    // rows per output, first row - start - MID, start, falling input order
 };
 
-// Two float32 operations per instruction (packed FMA / multiply of sm_100 on).
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<unsigned long long &>(d))
-        : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)),
-          "l"(reinterpret_cast<unsigned long long &>(c)));
-    return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;"
-        : "=l"(reinterpret_cast<unsigned long long &>(d))
-        : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
-    return d;
-}
-
-// *p (shared memory) where w > 0, else 0, without reading: lanes that read
-// nothing cause no bank conflicts
-__device__ __forceinline__ float lds_if(const float *p, float w) {
-    float x = 0.f;
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.gt.f32 q, %2, 0f00000000;\n\t@q ld.shared.f32 %0, [%1];\n\t}"
-                 : "+f"(x)
-                 : "r"((unsigned)__cvta_generic_to_shared(p)), "f"(w));
-    return x;
-}
-
 // One line and view of a warp.  VEC: floats per input load (4 needs input
 // columns that start on 16-byte boundaries).  M = 2 takes outputs of up to 2
 // rows, M = 1 of up to 4.
@@ -289,8 +262,7 @@ struct Strip {
     }
 
     __device__ __forceinline__ void load(unsigned j, float2 (&r)[2]) const {  // of input column j
-        const char *q;  // in + j * st, as one instruction
-        asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(q) : "r"(j), "r"(st), "l"(in));
+        const char *q = ptr_at(in, j, st);
         if (VEC == 4) {
             const float4 f = __ldg(reinterpret_cast<const float4 *>(q));
             r[0] = make_float2(f.x, f.y);
@@ -302,12 +274,12 @@ struct Strip {
         }
     }
     static __device__ __forceinline__ void mul(float x, const float2 (&r)[2], float2 (&o)[2]) {
-        o[0] = mul2(make_float2(x, x), r[0]);
-        o[1] = mul2(make_float2(x, x), r[1]);
+        o[0] = pk_mul(make_float2(x, x), r[0]);
+        o[1] = pk_mul(make_float2(x, x), r[1]);
     }
     static __device__ __forceinline__ void mac(float x, const float2 (&r)[2], float2 (&o)[2]) {
-        o[0] = fma2(make_float2(x, x), r[0], o[0]);
-        o[1] = fma2(make_float2(x, x), r[1], o[1]);
+        o[0] = pk_fma(make_float2(x, x), r[0], o[0]);
+        o[1] = pk_fma(make_float2(x, x), r[1], o[1]);
     }
     __device__ __forceinline__ void put(int lane, float *t, const float2 (&o)[2]) const {
         if (VEC == 4) {
@@ -328,11 +300,11 @@ struct Strip {
         for (int m = 0; m + 1 < M; m += 2) {
             const float *t0 = T + q[m], *t1 = T + q[m + 1];
             float2 a = make_float2(grp[m], grp[m + 1]);
-            a = fma2(make_float2(w[m][0], w[m + 1][0]), make_float2(t0[0], t1[0]), a);
-            a = fma2(make_float2(w[m][1], w[m + 1][1]), make_float2(t0[1], t1[1]), a);
+            a = pk_fma(make_float2(w[m][0], w[m + 1][0]), make_float2(t0[0], t1[0]), a);
+            a = pk_fma(make_float2(w[m][1], w[m + 1][1]), make_float2(t0[1], t1[1]), a);
             if (!two) {  // a third row is read only by the outputs that have one
                 const float2 x = make_float2(lds_if(t0 + 2, w[m][2]), lds_if(t1 + 2, w[m + 1][2]));
-                a = fma2(make_float2(w[m][2], w[m + 1][2]), x, a);
+                a = pk_fma(make_float2(w[m][2], w[m + 1][2]), x, a);
             }
             grp[m] = a.x;
             grp[m + 1] = a.y;

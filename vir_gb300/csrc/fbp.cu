@@ -34,13 +34,6 @@ namespace cg = cooperative_groups;
 // added in rank order through distributed shared memory.
 constexpr int PX = 2, VB = 256;
 
-// 1 / d to about half an ulp: the hardware's estimate and one Newton step.
-__device__ __forceinline__ float recip(float d) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    return fmaf(fmaf(-d, r, 1.0f), r, r);
-}
-
 template <bool FAN>
 __global__ void __launch_bounds__(256)
 fbp2d_bp_kernel(vg_dd2d_geom g, const float *__restrict__ q, const double *__restrict__ trig, float scale,
@@ -83,7 +76,7 @@ fbp2d_bp_kernel(vg_dd2d_geom g, const float *__restrict__ q, const double *__res
             for (int i = 0; i < PX; ++i) {
                 float p = fmaf(-cs.y, x[i], py), w = 1.0f;
                 if (FAN) {
-                    const float r = recip(fmaf(-cs.x, x[i], dy));
+                    const float r = recip_n(fmaf(-cs.x, x[i], dy));
                     p *= r;
                     w = (g.DSO * r) * (g.DSO * r);  // 1 / U^2
                 }

@@ -35,15 +35,17 @@
 //    more than 64, take a per-cell path.
 //  BP (sf3d_bp_kernel): the sinogram is first multiplied by l_theta
 //    (sf3d_weight, into the workspace, a chunk of views at a time); block =
-//    8 x 8 columns x 32 slices, thread = one slice of 8 columns; per view a
-//    table of the columns' u cells and F1 l_phi0 weights (at most 4 u cells
-//    per column, else a per-voxel path), then each voxel gathers its 1-3 v
-//    cells x 4 u cells.
+//    8 x 8 columns x 32 or 64 slices, warp = 8 columns; the two footprints are
+//    applied one after the other, see there.
+#include <cooperative_groups.h>
+#include <math.h>
+
 #include "vg_common.cuh"
 
 namespace {
 
 using namespace vg;
+namespace cg = cooperative_groups;
 
 __device__ __forceinline__ float2 view_cs(const double *__restrict__ trig, int ia) {
     return make_float2((float)__ldg(trig + 2 * ia), (float)__ldg(trig + 2 * ia + 1));
@@ -420,13 +422,26 @@ __global__ void sf3d_weight(vg_dd3d_geom g, const float *__restrict__ sino, int 
     }
 }
 
-constexpr int BT = 8, BZ = 32, BKU = 4;
+// The footprints are applied one after the other.  A warp owns 8 columns and
+// 32 M slices of each, and walks the views, 4 at a time (their F1 l_phi0 weights
+// and v maps tabulated at once, lane = view x column).  Per column and view it
+//   u: adds the 1-4 u cells under the column, times F1 l_phi0, over the window of
+//      v cells its slices project to (16-byte loads, lane = 4 cells), into a row
+//      buffer in shared memory;
+//   v: lets every slice add its 2-5 cells of the buffer with their overlaps.
+// Overlaps are in cell units, counted from about the window's middle.  Sums: 16
+// views in registers, then a compensated sum per voxel in shared memory.
+// Columns over more than 4 u cells, or whose slices reach more cells than the
+// buffer holds, take a per-voxel path.  With too few tiles to fill the GPU the
+// blocks of a cluster share a tile's views; sums meet in rank order.
+constexpr int BT = 8, BKU = 4;
+constexpr int BW = 128, MID = 40;  // cells of a row buffer, and where their count starts
+constexpr int BP_GROUP = 16;
 
-struct SfBpTab {
-    float4 w[2][BT * BT];   // F1 l_phi0 of u cells j0 .. j0 + 3
-    int j0[2][BT * BT];
-    float mz[2][BT * BT];
-    int wide[2];
+struct SfBpWarp {
+    float T[2][2][BW];
+    float4 w[4][BT];    // F1 l_phi0 / dv of u cells j0 .. j0 + 3
+    float4 rec[4][BT];  // v cells per slice, first cell - start - MID, start, j0 | count << 21
 };
 
 // one voxel, one view, straight from the weighted sinogram (any geometry)
@@ -454,110 +469,261 @@ __device__ __noinline__ float sf_voxel_view(const vg_dd3d_geom &g, const float *
     return part * inv_dv;
 }
 
-// the 8 voxels x0 .. x0 + 7 of row iy, slice iz (0 beyond the volume)
-__device__ __noinline__ void sf_voxels_view(const vg_dd3d_geom &g, const float *__restrict__ q, float c,
-                                            float s, int x0, int iy, int iz, float *out) {
-    for (int i = 0; i < BT; ++i) {
-        const int ix = x0 + i;
-        out[i] = ix < g.nx ? sf_voxel_view(g, q, c, s, vox(g.d_pix, ix, g.nx), vox(g.d_pix, iy, g.ny), iz)
-                           : 0.f;
-    }
-}
+constexpr int SF_BP_MINB = 3;
 
-__global__ void __launch_bounds__(256, 4)
+template <int VEC, int M>
+__global__ void __launch_bounds__(256, SF_BP_MINB)
 sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__restrict__ trig, int a0,
                int cnt, int accumulate, float *__restrict__ vol) {
-    __shared__ SfBpTab T;
-    const int z0 = blockIdx.x * BZ, y0 = blockIdx.y * BT, x0 = blockIdx.z * BT;
+    constexpr int SZ = 32 * M, NW = M == 2 ? 3 : 5, NV = 4 / VEC;
+    extern __shared__ float4 smem4[];
+    float2 *kh = reinterpret_cast<float2 *>(smem4);  // [BT * BT][SZ] (sum, compensation)
+    cg::cluster_group cl = cg::this_cluster();
+    const int S = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int z0 = (blockIdx.x / S) * SZ, y0 = blockIdx.y * BT, x0 = blockIdx.z * BT;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int iz = z0 + lane, iy = y0 + warp;
-    const float inv_du = 1.0f / g.du, inv_dv = 1.0f / g.dv;
-    const float U0 = uedge(g, 0), V0 = vedge(g, 0);
-    const float hz = 0.5f * g.nz;
-    Kahan acc[BT];
-    float grp[BT];
-#pragma unroll
-    for (int i = 0; i < BT; ++i) grp[i] = 0.f;
-    int ngrp = 0;
-    // T.wide[b] == a marks view a for the per-voxel path; writers only ever
-    // store that marker, so no reset races with them
-    if (tid < 2) T.wide[tid] = -1;
+    SfBpWarp &W = reinterpret_cast<SfBpWarp *>(kh + BT * BT * SZ)[warp];
+    const int iy = y0 + warp, zn = min(SZ, g.nz - z0);
+    const float inv_du = 1.0f / g.du, U0 = uedge(g, 0);
+    const float zd = (float)z0 - 0.5f * g.nz;  // exact
+    const float cv = 0.5f * g.nv - g.sv, ci = floorf(cv), cf = cv - ci;  // cell coordinate of v = 0
+    for (int c = warp; c < BT * BT; c += 8)
+        for (int m = 0; m < M; ++m) kh[c * SZ + 32 * m + lane] = make_float2(0.f, 0.f);
     __syncthreads();
-    for (int a = 0; a < cnt; ++a) {
-        const int b = a & 1;
-        const float2 cs = view_cs(trig, a0 + a);
-        if (tid < BT * BT) {
-            const int ix = x0 + (tid & 7), jy = y0 + (tid >> 3);
-            float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-            int j0 = 0;
-            float mz = 1.f;
-            if (ix < g.nx && jy < g.ny) {
-                const SfCol C = sf_col(g, cs.x, cs.y, vox(g.d_pix, ix, g.nx), vox(g.d_pix, jy, g.ny));
+    float grp[BT][M];
+#pragma unroll
+    for (int c = 0; c < BT; ++c)
+#pragma unroll
+        for (int m = 0; m < M; ++m) grp[c][m] = 0.f;
+    int ngrp = 0;
+    auto flush = [&]() {
+#pragma unroll
+        for (int c = 0; c < BT; ++c)
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                float2 *k = kh + (c + BT * warp) * SZ + 32 * m + lane;
+                Kahan a;
+                a.s = k->x; a.c = k->y;
+                a.add(grp[c][m]);
+                *k = make_float2(a.s, a.c);
+                grp[c][m] = 0.f;
+            }
+        ngrp = 0;
+    };
+    const int va0 = (int)((long long)cnt * rank / S), va1 = (int)((long long)cnt * (rank + 1) / S);
+    for (int ib = va0; ib < va1; ib += 4) {
+        unsigned slow, live;
+        {
+            const int sv = lane >> 3, c = lane & 7, ix = x0 + c;
+            const float2 cs = view_cs(trig, a0 + min(ib + sv, cnt - 1));
+            float w[BKU] = {0.f, 0.f, 0.f, 0.f};
+            float B = 1.f, first = 0.f;
+            int j0 = 0, n = 0, vs = 0;
+            bool far = false;
+            if (ix < g.nx && iy < g.ny) {
+                const SfCol C = sf_col(g, cs.x, cs.y, vox(g.d_pix, ix, g.nx), vox(g.d_pix, iy, g.ny));
                 const int ja = (int)floorf((C.t0 - U0) * inv_du), jb = (int)floorf((C.t3 - U0) * inv_du);
-                if (jb - ja >= BKU && jb >= 0 && ja < g.nu) T.wide[b] = a;
-                j0 = ja;
-                float ww[BKU];
+                j0 = min(max(ja, 0), g.nu - 1);
+                n = max(min(jb, g.nu - 1) - max(ja, 0) + 1, 0);
+                if (jb - ja >= BKU) n = n > 0 ? BKU + 1 : 0;
+                float e = trap_cum(uedge(g, j0), C);
+                const float f = inv_du * C.lphi;
 #pragma unroll
                 for (int t = 0; t < BKU; ++t) {
-                    const int j = ja + t;
-                    ww[t] = (j >= 0 && j < g.nu && j <= jb)
-                        ? uweight(C, uedge(g, j), uedge(g, j + 1), inv_du) : 0.f;
+                    const float h = trap_cum(uedge(g, j0 + t + 1), C);
+                    w[t] = t < n ? (h - e) * f : 0.f;
+                    e = h;
                 }
-                w = make_float4(ww[0], ww[1], ww[2], ww[3]);
-                mz = C.mz;
+                B = C.mz / g.dv;
+                const float t = B * zd, tf = floorf(t);
+                const int fl = (int)tf + (int)ci;
+                vs = VEC == 4 ? fl & ~3 : fl;
+                first = (t - tf) + cf + (float)(fl - vs - MID);
+                const int ve = vs + __float2int_rd(fmaf(B, (float)zn, first)) + MID + 1;
+                far = ve <= 0 || vs >= g.nv;
+                if (B > NW - 1.0f || ve - vs > BW - NW + 1) n = n > 0 ? BKU + 1 : 0;
             }
-            T.w[b][tid] = w;
-            T.j0[b][tid] = j0;
-            T.mz[b][tid] = mz;
+            if (far) n = 0;
+            slow = __ballot_sync(0xffffffffu, n > BKU);
+            live = __ballot_sync(0xffffffffu, n > 0);
+            W.w[sv][c] = make_float4(w[0], w[1], w[2], w[3]);
+            W.rec[sv][c] = make_float4(B, first, __int_as_float(vs), __int_as_float(j0 | n << 21));
+            __syncwarp();
         }
-        __syncthreads();
-        const float *q = qw + (size_t)a * g.nu * g.nv;
-        if (iy < g.ny && iz < g.nz) {
-            if (T.wide[b] != a) {
+        const int nb = min(4, va1 - ib);
+        for (int sv = 0; sv < nb; ++sv) {
+            const unsigned lv = live >> (8 * sv) & 0xff, sl = slow >> (8 * sv) & 0xff;
+            const char *q = reinterpret_cast<const char *>(qw + (size_t)(ib + sv) * g.nu * g.nv);
 #pragma unroll
-                for (int i = 0; i < BT; ++i) {
-                    const int col = i + BT * warp;
-                    const float mz = T.mz[b][col];
-                    const float4 w = T.w[b][col];
-                    const int j0 = T.j0[b][col];
-                    const float va = mz * ((float)iz - hz), vb = va + mz;
-                    const int la = max((int)floorf((va - V0) * inv_dv), 0);
-                    const int lb = min((int)floorf((vb - V0) * inv_dv), g.nv - 1);
-                    const float wt[BKU] = {w.x, w.y, w.z, w.w};
-                    float part = 0.f;
-                    for (int l = la; l <= lb; ++l) {
-                        const float ov = fminf(vb, vedge(g, l + 1)) - fmaxf(va, vedge(g, l));
-                        if (ov <= 0.f) continue;
-                        float r = 0.f;
+            for (int c0 = 0; c0 < BT; c0 += 2) {
+                if (!(lv >> c0 & 3)) continue;
+                if (sl >> c0 & 3) {
+                    const float2 cs = view_cs(trig, a0 + ib + sv);
 #pragma unroll
-                        for (int t = 0; t < BKU; ++t)
-                            if (wt[t] != 0.f) r = fmaf(wt[t], __ldg(q + (size_t)(j0 + t) * g.nv + l), r);
-                        part = fmaf(r, ov, part);
+                    for (int c = c0; c < c0 + 2; ++c)
+#pragma unroll
+                        for (int m = 0; m < M; ++m) {
+                            const int iz = z0 + 32 * m + lane;
+                            if (x0 + c < g.nx && iz < g.nz)
+                                grp[c][m] += sf_voxel_view(g, reinterpret_cast<const float *>(q), cs.x, cs.y,
+                                                           vox(g.d_pix, x0 + c, g.nx),
+                                                           vox(g.d_pix, iy, g.ny), iz);
+                        }
+                    continue;
+                }
+                float (*T)[BW] = W.T[c0 >> 1 & 1];
+                float wv[2][M][NW];
+                int qi[2][M];
+                bool two[2];
+                float2 o[2][2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float4 w = W.w[sv][c0 + h], rc = W.rec[sv][c0 + h];
+                    const int vs = __float_as_int(rc.z), bits = __float_as_int(rc.w), n = bits >> 21;
+                    const unsigned j = bits & 0x1fffff;  // nu < 2^21
+                    const int win = __float2int_rd(fmaf(rc.x, (float)zn, rc.y)) + MID + NW;
+                    // this lane's cells, clamped to the window and the detector
+                    int vo[NV];
+#pragma unroll
+                    for (int i = 0; i < NV; ++i) {
+                        const int v = vs + min(VEC == 4 ? 4 * lane : lane + 32 * i, (win - 1) & ~(VEC - 1));
+                        vo[i] = 4 * min(max(v, 0), g.nv - VEC);
                     }
-                    grp[i] = fmaf(part, inv_dv, grp[i]);
+                    const char *p = VEC == 4 ? q + vo[0] : q;
+                    auto load = [&](unsigned jj, float2 (&r)[2]) {
+                        const char *a = ptr_at(p, jj, 4u * g.nv);
+                        if (VEC == 4) {
+                            const float4 f = __ldg(reinterpret_cast<const float4 *>(a));
+                            r[0] = make_float2(f.x, f.y);
+                            r[1] = make_float2(f.z, f.w);
+                        } else {
+                            auto at = [&](int i) {
+                                return __ldg(reinterpret_cast<const float *>(a + vo[i & (NV - 1)]));
+                            };
+                            r[0] = make_float2(at(0), at(1));
+                            if (win > 64) r[1] = make_float2(at(2), at(3));
+                        }
+                    };
+                    float2 r0[2], r1[2], r2[2];
+                    load(j, r0);
+                    load(j + (n > 1), r1);
+                    load(j + (n > 2 ? 2 : n > 1 ? 1 : 0), r2);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        o[h][i] = pk_fma(dup(w.z), r2[i], pk_fma(dup(w.y), r1[i], pk_mul(dup(w.x), r0[i])));
+                    if (n > 3) {
+                        load(j + 3, r0);
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) o[h][i] = pk_fma(dup(w.w), r0[i], o[h][i]);
+                    }
+                    if (n == 0) o[h][0] = o[h][1] = dup(0.f);  // nothing from its nearest u cell
+                    // overlaps of this lane's slices with their cells
+                    float over = 0.f;
+                    int qf[M];
+#pragma unroll
+                    for (int m = 0; m < M; ++m) {
+                        const float zm = (float)(32 * m + lane);
+                        const float tl = fmaf(rc.x, zm, rc.y), th = fmaf(rc.x, zm + 1.0f, rc.y);
+                        const float tf = floorf(tl);
+                        wv[h][m][0] = fminf(th, tf + 1.0f) - tl;
+#pragma unroll
+                        for (int t = 1; t < NW; ++t) wv[h][m][t] = __saturatef(th - (tf + (float)t));
+                        if (32 * m + lane < zn) over = fmaxf(over, th - tf);
+                        qf[m] = (int)tf + MID;
+                        qi[h][m] = min(qf[m], BW - NW);  // slices past the volume read anything
+                    }
+                    two[h] = !__any_sync(0xffffffffu, over > 2.0f);
+                    if (vs < 0 || vs + win > g.nv) {
+#pragma unroll
+                        for (int m = 0; m < M; ++m)
+#pragma unroll
+                            for (int t = 0; t < NW; ++t)
+                                if ((unsigned)(qf[m] + vs + t) >= (unsigned)g.nv) wv[h][m][t] = 0.f;
+                    }
+                    if (VEC == 4) {
+                        if (4 * lane < win)
+                            *reinterpret_cast<float4 *>(T[h] + 4 * lane) =
+                                make_float4(o[h][0].x, o[h][0].y, o[h][1].x, o[h][1].y);
+                    } else {
+                        T[h][lane] = o[h][0].x;
+                        T[h][lane + 32] = o[h][0].y;
+                        if (win > 64) {
+                            T[h][lane + 64] = o[h][1].x;
+                            T[h][lane + 96] = o[h][1].y;
+                        }
+                    }
                 }
-            } else {
-                float wv[BT];
-                sf_voxels_view(g, q, cs.x, cs.y, x0, iy, iz, wv);
+                __syncwarp();
 #pragma unroll
-                for (int i = 0; i < BT; ++i) grp[i] += wv[i];
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int m = 0; m < M; ++m) {
+                        const float *t = T[h] + qi[h][m];
+                        float a = grp[c0 + h][m];
+                        a = fmaf(wv[h][m][0], t[0], a);
+                        a = fmaf(wv[h][m][1], t[1], a);
+                        if (!two[h]) {
+#pragma unroll
+                            for (int i = 2; i < NW; ++i)
+                                a = fmaf(wv[h][m][i], lds_if(t + i, wv[h][m][i]), a);
+                        }
+                        grp[c0 + h][m] = a;
+                    }
             }
+            if (++ngrp == BP_GROUP) flush();
         }
-        if (++ngrp == 16) {
+        __syncwarp();  // the table and the row buffers are reused
+    }
+    flush();
+    if (S > 1) cl.sync();
+    else __syncthreads();
+    for (int col = warp * S + rank; col < BT * BT; col += 8 * S) {
+        const int ix = x0 + (col & 7), jy = y0 + (col >> 3);
+        if (ix >= g.nx || jy >= g.ny) continue;
 #pragma unroll
-            for (int i = 0; i < BT; ++i) { acc[i].add(grp[i]); grp[i] = 0.f; }
-            ngrp = 0;
+        for (int m = 0; m < M; ++m) {
+            const int iz = 32 * m + lane;
+            if (iz >= zn) continue;
+            float2 *k = kh + col * SZ + iz;
+            Kahan a;
+            if (S == 1) {
+                a.s = k->x;
+            } else {
+                for (int r = 0; r < S; ++r) {
+                    const float2 t = *cl.map_shared_rank(k, r);
+                    a.add(t.x);
+                    a.add(-t.y);
+                }
+            }
+            float *o = vol + ((size_t)ix * g.ny + jy) * g.nz + z0 + iz;
+            *o = accumulate ? *o + a.s : a.s;
         }
     }
-    if (iy >= g.ny || iz >= g.nz) return;
-#pragma unroll
-    for (int i = 0; i < BT; ++i) {
-        const int ix = x0 + i;
-        if (ix >= g.nx) continue;
-        acc[i].add(grp[i]);
-        float *o = vol + ((size_t)ix * g.ny + iy) * g.nz + iz;
-        *o = accumulate ? *o + acc[i].s : acc[i].s;
-    }
+    if (S > 1) cl.sync();  // no block leaves while its sums are read
+}
+
+template <int VEC, int M>
+int launch_bp(const vg_dd3d_geom *g, const float *qw, const double *trig, int a0, int cnt, float *vol,
+              cudaStream_t st) {
+    constexpr size_t smem = (size_t)BT * BT * 32 * M * sizeof(float2) + 8 * sizeof(SfBpWarp);
+    const long long tiles = (long long)ceil_div(g->nz, 32 * M) * ceil_div(g->ny, BT) * ceil_div(g->nx, BT);
+    int S = 1;
+    while (S < 8 && tiles * S < 3 * 152 && cnt >= 32 * S) S *= 2;
+    int s = cuda_status(cudaFuncSetAttribute(sf3d_bp_kernel<VEC, M>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "sf3d_bp");
+    if (s) return s;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(ceil_div(g->nz, 32 * M) * S, ceil_div(g->ny, BT), ceil_div(g->nx, BT));
+    c.blockDim = dim3(256);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return cuda_status(cudaLaunchKernelEx(&c, sf3d_bp_kernel<VEC, M>, *g, qw, trig, a0, cnt, (int)(a0 > 0), vol),
+                       "sf3d_bp");
 }
 
 int check(const vg_dd3d_geom *g) {
@@ -637,14 +803,19 @@ extern "C" int vg_sf3d_bp(const vg_dd3d_geom *g, const float *sino, const double
                "sf3d_bp: workspace of %zu bytes needed (vg_sf3d_workspace_bytes)", need);
     cudaStream_t s = as_stream(stream);
     float *qw = static_cast<float *>(workspace);
-    dim3 grid(ceil_div(g->nz, BZ), ceil_div(g->ny, BT), ceil_div(g->nx, BT));
+    // 64 slices per warp while the cells they project to fit a row buffer, by the
+    // largest magnification in the volume; 16-byte loads where rows are aligned
+    const double r = 0.5 * hypot((double)g->nx, (double)g->ny) * g->d_pix;
+    const double bmax = g->DSD / (g->DSO - fmin(r, 0.999 * g->DSO)) * g->d_pix / g->dv;
+    const bool m2 = g->nz > 32 && 64.0 * bmax + 9.0 <= BW;
+    const bool vec = g->nv % 4 == 0 && ((uintptr_t)qw & 15) == 0;
+    auto bp = m2 ? (vec ? launch_bp<4, 2> : launch_bp<1, 2>) : (vec ? launch_bp<4, 1> : launch_bp<1, 1>);
     for (int a0 = 0; a0 < g->na; a0 += (int)nch) {
         const int cnt = (int)((size_t)(g->na - a0) < nch ? (size_t)(g->na - a0) : nch);
         sf3d_weight<<<1216, 256, 0, s>>>(*g, sino, a0, cnt, qw);
         st = launch_status("sf3d_weight");
         if (st) return st;
-        sf3d_bp_kernel<<<grid, 256, 0, s>>>(*g, qw, trig, a0, cnt, a0 > 0, vol);
-        st = launch_status("sf3d_bp");
+        st = bp(g, qw, trig, a0, cnt, vol, s);
         if (st) return st;
     }
     return VG_OK;
