@@ -375,8 +375,7 @@ int vg_dd3d_bp(const vg_dd3d_geom *g, const float *sino, const double *trig,
  * through the column centre, l_theta = sqrt(1 + v^2 / (u^2 + DSD^2)) at the
  * cell centre.
  * vg_sf3d_fp: sino (na, nu, nv) = the line integrals above, gather form;
- *   workspace: the volume's per-column running sums over z (nx ny (nz + 1)
- *   floats, FP64-accumulated) from which each column's v profile is read.
+ *   workspace: nx ny (nz + 1) floats, checked but not used.
  * vg_sf3d_bp: vol = its exact adjoint; workspace: the l_theta-weighted
  *   sinogram of a chunk of views (at most 256 MiB or one view).
  * Both take vg_sf3d_workspace_bytes(g) bytes (the larger need), 4-byte

@@ -1,0 +1,59 @@
+"""The cone SF pair's column kernels at the sizes where they change form: 1, 2 or
+3 groups of 32 outputs per warp, 16-byte and 4-byte loads, ragged tiles, columns
+over more than 4 u cells, lines of more than 32 columns under 8 u cells, windows
+longer than a row buffer, tiles shared by a cluster of blocks.
+
+Tolerance: the pair is held to 5e-5 of the largest value against the FP64 oracle
+elsewhere; the same here."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# shape, nu, nv, na, du, dv, d_pix, DSO, DSD
+CASES = {
+    "fp16_bp4": ((12, 9, 64), 21, 97, 5, 1.1, 1.3, 0.9, 40.0, 70.0),
+    "fp4_bp16": ((9, 12, 65), 17, 96, 5, 1.2, 1.2, 0.8, 40.0, 70.0),
+    "small": ((5, 3, 31), 7, 30, 7, 1.0, 1.0, 1.0, 30.0, 50.0),
+    "thin": ((8, 9, 70), 14, 40, 5, 0.9, 2.1, 0.5, 40.0, 70.0),
+    "wide_bp": ((7, 8, 33), 60, 50, 4, 0.3, 0.5, 1.0, 30.0, 55.0),
+    "wide_fp": ((40, 44, 6), 9, 12, 4, 11.0, 2.0, 1.0, 60.0, 100.0),
+    "tall": ((6, 7, 200), 12, 20, 4, 1.5, 8.0, 0.5, 40.0, 70.0),
+    "views": ((8, 8, 12), 14, 12, 130, 1.0, 1.5, 1.0, 30.0, 50.0),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_sf_cone_columns_vs_oracle(vg, orc, name):
+    from vir_gb300.sys_mat import sp
+    shape, nu, nv, na, du, dv, d, DSO, DSD = CASES[name]
+    rng = np.random.default_rng(23)
+    angs = np.linspace(0.03, 0.03 + 2 * np.pi, na, endpoint=False)
+    f = lambda v: float(np.float32(v))
+    kw = dict(du=f(du), dv=f(dv), su=f(0.3), sv=f(-0.4), d_pix=f(d))
+    vol = rng.random(shape).astype(np.float32)
+    y = rng.random((na, nu, nv)).astype(np.float32)
+    for got, ref in ((sp.sf_fp_cone_3d(vol, angs, nu, nv, DSO, DSD, **kw),
+                      orc.sf_fp_cone_3d(vol, angs, nu, nv, DSO, DSD, **kw)),
+                     (sp.sf_bp_cone_3d(y, angs, shape, DSO, DSD, **kw),
+                      orc.sf_bp_cone_3d(y, angs, shape, DSO, DSD, **kw))):
+        assert np.abs(got - ref).max() <= 5e-5 * np.abs(ref).max()
+
+
+def test_sf_cone_columns_nan_stays_near(vg):
+    """A NaN voxel or cell reaches only outputs within two of those it overlaps."""
+    import torch
+    from vir_gb300.sys_mat import sp
+    shape, nu, nv, na = (16, 16, 32), 40, 64, 6
+    angs = np.linspace(0.1, 0.1 + 2 * np.pi, na, endpoint=False)
+    kw = dict(du=1.0, dv=1.0, d_pix=1.0)
+    for call, size in ((lambda t: sp.sf_fp_cone_3d(t, angs, nu, nv, 60.0, 100.0, **kw), shape),
+                       (lambda t: sp.sf_bp_cone_3d(t, angs, shape, 60.0, 100.0, **kw), (na, nu, nv))):
+        a = torch.rand(size, generator=torch.Generator().manual_seed(2)).cuda()
+        hit = torch.zeros_like(a)
+        hit.view(-1)[a.numel() // 2 + 7] = 1.0
+        near = (call(hit) != 0).float()
+        near = (torch.nn.functional.max_pool2d(near[:, None], 5, 1, 2)[:, 0] if size == shape
+                else torch.nn.functional.max_pool3d(near[None, None], 5, 1, 2)[0, 0]) > 0
+        a.view(-1)[a.numel() // 2 + 7] = float("nan")
+        assert not bool((torch.isnan(call(a)) & ~near).any())

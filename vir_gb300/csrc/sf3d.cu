@@ -22,17 +22,8 @@
 // The forward projection returns these line integrals; the back projection
 // is its exact adjoint (vir has no back projector for this footprint).
 //
-//  FP (sf3d_zprefix, sf3d_fp_kernel): the volume's per-column running sums
-//    over z are formed first (workspace).  Block = (view, 32 u x 64 v cells),
-//    thread = 4 u cells (warp) x 2 v cells (lanes).  For each orthogonal
-//    pixel line whose columns reach the tile, the block tabulates in shared
-//    memory the columns' footprints, the covering columns and F1 weights of
-//    each u cell, and each column's v profile over the tile's v cells
-//    g(c, l) = sum_z f(c, z) F2(l; c, z) as the running integral at the 65
-//    v edges (the z sums interpolated at the edge's slice coordinate); each
-//    cell then adds F1 * l_phi0 * (difference of its edges) over its 1-8
-//    covering columns.  Lines where a u cell meets more columns, or the tile
-//    more than 64, take a per-cell path.
+//  FP (sf3d_fp_kernel): warp = 8 u cells x 32-96 v cells of one view; walks the
+//    lines and, on each, the columns that cover its cells, see there.
 //  BP (sf3d_bp_kernel): the sinogram is first multiplied by l_theta
 //    (sf3d_weight, into the workspace, a chunk of views at a time); block =
 //    8 x 8 columns x 32 or 64 slices, warp = 8 columns; the two footprints are
@@ -100,22 +91,15 @@ __device__ __forceinline__ SfCol sf_col(const vg_dd3d_geom &g, float c, float s,
     return C;
 }
 
-// Integral of the unit trapezoid (t0, t1, t2, t3) from -inf to u.
+// Integral of the unit trapezoid (t0, t1, t2, t3) from -inf to u: the parts of
+// the rise, the top and the fall before u (no branches: lanes hold footprints
+// at all stages).
 __device__ __forceinline__ float trap_cum(float u, const SfCol &C) {
-    if (u <= C.t0) return 0.f;
-    const float a = 0.5f * (C.t1 - C.t0);
-    if (u <= C.t1) {
-        const float e = u - C.t0;
-        return __fdividef(e * e, 2.f * (C.t1 - C.t0));
-    }
-    if (u <= C.t2) return a + (u - C.t1);
-    const float b = a + (C.t2 - C.t1);
-    const float r = 0.5f * (C.t3 - C.t2);
-    if (u <= C.t3) {
-        const float e = C.t3 - u;
-        return b + r - __fdividef(e * e, 2.f * (C.t3 - C.t2));
-    }
-    return b + r;
+    const float a = fminf(fmaxf(u, C.t0), C.t1) - C.t0, b = fminf(fmaxf(u, C.t1), C.t2) - C.t1;
+    const float f = C.t3 - C.t2, e = C.t3 - fminf(fmaxf(u, C.t2), C.t3);
+    const float rise = __fdividef(a * a, fmaxf(2.f * (C.t1 - C.t0), 1e-30f));
+    const float fall = 0.5f * f - __fdividef(e * e, fmaxf(2.f * f, 1e-30f));
+    return rise + b + fall;
 }
 
 // F1 averaged over [ua, ub] (cell width du), times l_phi0
@@ -150,48 +134,34 @@ __device__ __forceinline__ float unproj_idx(const vg_dd3d_geom &g, float c, floa
     return __fdividef(b, g.d_pix) + 0.5f * nd;
 }
 
-// Per-column running sums over z for the forward projection's v profiles:
-// zp[c][z] = sum_{z' < z} f(c, z') for z = 0 .. nz (column c = x ny + y),
-// accumulated in FP64 and rounded once, so that a profile's edge value
-// (an interpolation of zp) and the difference of two of them carry a
-// rounding of the column's total, not of its summation.  One warp per column.
-__global__ void __launch_bounds__(256)
-sf3d_zprefix(vg_dd3d_geom g, const float *__restrict__ vol, float *__restrict__ zp) {
-    const size_t col = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (col >= (size_t)g.nx * g.ny) return;
-    const float *f = vol + col * g.nz;
-    float *p = zp + col * (g.nz + 1);
-    if (lane == 0) p[0] = 0.f;
-    double carry = 0.0;
-    for (int z0 = 0; z0 < g.nz; z0 += 32) {
-        const int z = z0 + lane;
-        double v = z < g.nz ? (double)__ldg(f + z) : 0.0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double t = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o) v += t;
-        }
-        if (z < g.nz) p[z + 1] = (float)(carry + v);
-        carry += __shfl_sync(0xffffffffu, v, 31);
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Forward projection
 // ---------------------------------------------------------------------------
-constexpr int SU = 32, SV = 64, SCMAX = 64, SKMAX = 8, SLINES = 2048;
+// A warp owns 8 u cells x 32 M v cells of one view and walks the orthogonal
+// lines of the volume.  The ranges of columns that reach its u cells are found
+// 32 lines at a time (lane = line), a line's footprints, F1 l_phi0 weights on
+// the 8 cells and v maps 32 columns at a time (lane = column).  Then per column
+// that covers any of the cells: its slices under the tile's v cells go to shared
+// memory (one 16-byte load per 4 slices, the next column's issued before this
+// one is used), every lane sums its M v cells' 2-5 slices with their overlaps,
+// and adds the result to the cells the column covers.  Overlaps are counted in
+// slices from about the window's middle.  Lines with more than 32 columns, or
+// v cells over more slices than a row buffer holds, take a per-cell path.  Sums:
+// 16 lines in registers, then a second running sum in shared memory.
+//
+// Bound by instruction issue (72 %, 213 per column and line for 8 x 96 cells).
+// 256^3, 360 views of 512 x 384: 55.3 -> 21.6 ms against profiles of every column
+// in block-wide tables, one barrier per line (144 instructions per 32 cells and
+// line); the weights by branches per lane and the FMAs by cell 28 ms.  4 blocks
+// per SM 21.6, 5 22.5, 6 22.4 ms.
+constexpr int SFW = 4, SF_FP_MINB = 4;  // warps per block
+constexpr int UC = 8;                   // u cells per warp
+constexpr int BW = 128, MID = 40;       // entries of a row buffer, and where their count starts
 
-// per-line tables, double-buffered by line parity
-struct SfFpTab {
-    SfCol col[2][SCMAX];
-    int poff[2][SCMAX];     // index of (column, z = 0) in the z-prefix array
-    int cf[2][SU], cn[2][SU];  // covering columns (table index, count) per u cell
-    float w[2][SU][SKMAX];  // F1 l_phi0 weights of those columns
-    float gv[2][SCMAX][SV + 1];  // per column: the v profile's running integral at the v edges
-    int2 kr[SLINES];        // per line: the range [x, y] of columns that can reach the tile
-    float ve[SV + 1];       // the tile's v cell edges
-    int wide[2];
+struct SfFpWarp {
+    float T[2][BW];
+    float w[32][UC];  // per column: F1 l_phi0 M d / dv on the u cells
+    float4 rec[32];   // slices per v cell, first slice - start - MID, start, index of the column
 };
 
 // one cell's share of one line, straight from global memory (any geometry)
@@ -215,193 +185,255 @@ __device__ __noinline__ float sf_cell_line(const vg_dd3d_geom &g, const float *_
     return part;
 }
 
-__global__ void __launch_bounds__(256, 3)
-sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const float *__restrict__ zp,
-               const double *__restrict__ trig, float *__restrict__ sino) {
-    __shared__ SfFpTab T;
-    const int ia = blockIdx.z;
-    const int u0 = blockIdx.y * SU, v0 = blockIdx.x * SV;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+template <int VEC, int M>
+__global__ void __launch_bounds__(32 * SFW, SF_FP_MINB)
+sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__restrict__ trig,
+               float *__restrict__ sino) {
+    constexpr int SZ = 32 * M, NW = M >= 2 ? 3 : 5;
+    extern __shared__ float4 smem4[];
+    const int ia = blockIdx.z, v0 = blockIdx.x * SZ;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int u0 = (blockIdx.y * SFW + warp) * UC;
+    SfFpWarp &W = reinterpret_cast<SfFpWarp *>(smem4)[warp];
+    float *acc = reinterpret_cast<float *>(reinterpret_cast<SfFpWarp *>(smem4) + SFW) + warp * UC * SZ + lane;
+    if (u0 >= g.nu) return;  // no block barriers below
     const float2 cs = view_cs(trig, ia);
     const float c = cs.x, s = cs.y;
     const bool xdrv = fabsf(s) >= fabsf(c);
     const int nd = xdrv ? g.nx : g.ny, no = xdrv ? g.ny : g.nx;
-    const float inv_du = 1.0f / g.du, inv_dv = 1.0f / g.dv;
-    const int nuT = min(SU, g.nu - u0), nvT = min(SV, g.nv - v0);
+    const float inv_du = 1.0f / g.du;
+    const int nuT = min(UC, g.nu - u0), zn = min(SZ, g.nv - v0);
     const float TUa = uedge(g, u0), TUb = uedge(g, u0 + nuT);
-    // the inverse edge map has a pole at u = -DSD pd / od; a tile holding it
-    // (or within two cells of it) cannot bound its columns through the map
+    // the inverse edge map has a pole at u = -DSD pd / od; cells holding it (or
+    // within two cells of it) cannot bound their columns through the map
     const float pd = xdrv ? -s : c, od = xdrv ? c : s;
-    bool tile_pole = false;
+    bool pole = false;
     if (od != 0.f) {
         const float up = -g.DSD * pd / od;
-        tile_pole = up >= TUa - 2.f * g.du && up <= TUb + 2.f * g.du;
+        pole = up >= TUa - 2.f * g.du && up <= TUb + 2.f * g.du;
     }
-    // this thread's (u cell, slot) in the weight table
-    const int wu = tid >> 3, wm = tid & 7;
-    float acc[8], grp[8];
+    const float kB = g.dv / (g.DSD * g.d_pix);  // slices per v cell = kB (DSO - o)
+    const float vd = (float)v0 - 0.5f * g.nv + g.sv;
+    const float ci = floorf(0.5f * g.nz), cf = 0.5f * g.nz - ci;
+    float2 grp[UC / 2][M];  // u cells in pairs
 #pragma unroll
-    for (int q = 0; q < 8; ++q) acc[q] = grp[q] = 0.f;
+    for (int q = 0; q < UC; ++q)
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            grp[q / 2][m] = dup(0.f);
+            acc[q * SZ + 32 * m] = 0.f;
+        }
     int ngrp = 0;
-    if (tid < 2) T.wide[tid] = -1;
-    if (tid <= SV) T.ve[tid] = vedge(g, v0 + tid);
-    const float hz = 0.5f * g.nz, nzf = (float)g.nz;
-    // columns of every line whose footprints can reach the tile, one line per
-    // thread: the map of the tile's u edges (widened by a cell) on both
-    // boundaries of the line, one column of margin each side
-    for (int jo = tid; jo < no; jo += 256) {
-        int kA = 0, kB = nd - 1;
-        if (!tile_pole) {
-            const float cj = vox(g.d_pix, jo, no), h = 0.5f * g.d_pix;
-            const float a0 = unproj_idx(g, c, s, xdrv, cj - h, TUa - g.du, nd);
-            const float a1 = unproj_idx(g, c, s, xdrv, cj + h, TUa - g.du, nd);
-            const float b0 = unproj_idx(g, c, s, xdrv, cj - h, TUb + g.du, nd);
-            const float b1 = unproj_idx(g, c, s, xdrv, cj + h, TUb + g.du, nd);
-            const float lo = fminf(fminf(a0, a1), fminf(b0, b1));
-            const float hi = fmaxf(fmaxf(a0, a1), fmaxf(b0, b1));
-            kA = max((int)floorf(fmaxf(lo, -2.f)) - 1, 0);
-            kB = min((int)floorf(fminf(hi, (float)nd + 2.f)) + 1, nd - 1);
-        }
-        T.kr[jo] = make_int2(kA, kB);
-    }
-    __syncthreads();
-    // phase 1 of a line: its columns' footprints and z-prefix rows into buffer bb
-    auto phase1 = [&](int io, int bb) {
-        const int2 kr = T.kr[io];
-        const int nk = kr.y - kr.x + 1;
-        if (nk <= SCMAX && tid < nk) {
-            const int k = kr.x + tid;
-            const float cen = vox(g.d_pix, io, no), bx = vox(g.d_pix, k, nd);
-            T.col[bb][tid] = sf_col(g, c, s, xdrv ? bx : cen, xdrv ? cen : bx);
-            const int ix = xdrv ? k : io, iy = xdrv ? io : k;
-            T.poff[bb][tid] = (ix * g.ny + iy) * (g.nz + 1);
-        }
-    };
-    auto next_line = [&](int io) {
-        do { ++io; } while (io < no && T.kr[io].x > T.kr[io].y);
-        return io;
-    };
-    // One barrier per line: the block builds line io's covering columns,
-    // weights and v profiles from buffer b together with the next line's
-    // footprints into buffer b ^ 1, then after the barrier each cell adds
-    // line io's columns.  Phase 3 of line io reads only phase-2 results of
-    // buffer b, which the block next writes two lines later, after the
-    // following line's barrier; T.wide[b] holds the index of the last wide
-    // line of buffer b (writers only store that index).
-    int io = next_line(-1), b = 0;
-    if (io < no) phase1(io, 0);
-    __syncthreads();
-    for (; io < no; b ^= 1) {
-        const int2 kr = T.kr[io];
-        const int kA = kr.x, kB = kr.y;
-        const int nk = kB - kA + 1;
-        const bool big = nk > SCMAX;
-        const int nxt = next_line(io);
-        if (nxt < no) phase1(nxt, b ^ 1);
-        if (!big) {
-            // phase 2a: covering columns of each u cell (the footprints move
-            // monotonically along the line, so they are consecutive; binary
-            // searches on the footprints' ends) and their weights, one
-            // (u cell, slot) per thread
-            if (wu < nuT) {
-                const float ua = uedge(g, u0 + wu), ub = uedge(g, u0 + wu + 1);
-                const bool inc = T.col[b][nk - 1].t0 >= T.col[b][0].t0;
-                // first covering: inc -> first t with t3 > ua; dec -> first t with t0 < ub
-                int lo = 0, hi = nk;
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    const bool past = inc ? (T.col[b][mid].t3 > ua) : (T.col[b][mid].t0 < ub);
-                    if (past) hi = mid; else lo = mid + 1;
-                }
-                const int first = lo;
-                // end (exclusive): inc -> first t with t0 >= ub; dec -> first t with t3 <= ua
-                lo = first; hi = nk;
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    const bool out = inc ? (T.col[b][mid].t0 >= ub) : (T.col[b][mid].t3 <= ua);
-                    if (out) hi = mid; else lo = mid + 1;
-                }
-                const int n = lo - first;
-                if (wm == 0) {
-                    T.cf[b][wu] = first;
-                    T.cn[b][wu] = min(n, SKMAX);
-                    if (n > SKMAX) T.wide[b] = io;
-                }
-                if (wm < n && wm < SKMAX) T.w[b][wu][wm] = uweight(T.col[b][first + wm], ua, ub, inv_du);
-            }
-            // phase 2b: per column, the running integral of its v profile at the
-            // tile's v edges: the column's z-prefix interpolated at the edge's
-            // slice coordinate s = v / (M d) + nz/2, times M d / dv; a cell's
-            // profile is the difference of its two edges
-            for (int p = tid; p < nk * (SV + 1); p += 256) {
-                const int t = p / (SV + 1), l = p - t * (SV + 1);
-                float e = 0.f;
-                if (l <= nvT) {
-                    const float sz = fminf(fmaxf(fmaf(T.ve[l], T.col[b][t].inv_mz, hz), 0.f), nzf);
-                    const float zf = fminf(floorf(sz), nzf - 1.f);
-                    const float *pc = zp + T.poff[b][t] + (int)zf;
-                    const float p0 = __ldg(pc), p1 = __ldg(pc + 1);
-                    e = fmaf(p1 - p0, sz - zf, p0) * (T.col[b][t].mz * inv_dv);
-                }
-                T.gv[b][t][l] = e;
+    for (int lb = 0; lb < no; lb += 32) {
+        // columns of line lb + lane whose footprints can reach the cells: the map of
+        // their outer edges (widened by a cell) on both boundaries of the line, one
+        // column of margin each side
+        int kA = 0, kE = -1;
+        if (lb + lane < no) {
+            kE = nd - 1;
+            if (!pole) {
+                const float cj = vox(g.d_pix, lb + lane, no), h = 0.5f * g.d_pix;
+                const float a0 = unproj_idx(g, c, s, xdrv, cj - h, TUa - g.du, nd);
+                const float a1 = unproj_idx(g, c, s, xdrv, cj + h, TUa - g.du, nd);
+                const float b0 = unproj_idx(g, c, s, xdrv, cj - h, TUb + g.du, nd);
+                const float b1 = unproj_idx(g, c, s, xdrv, cj + h, TUb + g.du, nd);
+                const float lo = fminf(fminf(a0, a1), fminf(b0, b1));
+                const float hi = fmaxf(fmaxf(a0, a1), fmaxf(b0, b1));
+                kA = max((int)floorf(fmaxf(lo, -2.f)) - 1, 0);
+                kE = min((int)floorf(fminf(hi, (float)nd + 2.f)) + 1, nd - 1);
             }
         }
-        __syncthreads();
-        // phase 3: each cell adds its covering columns' weighted profiles
-        float part[8];
-        if (!big && T.wide[b] != io) {
+        unsigned lines = __ballot_sync(0xffffffffu, kE >= kA);
+        while (lines) {
+            const int l = __ffs(lines) - 1, io = lb + l;
+            lines &= lines - 1;
+            const int ka = __shfl_sync(0xffffffffu, kA, l), ke = __shfl_sync(0xffffffffu, kE, l);
+            bool slow = ke - ka >= 32;
+            unsigned cols = 0;
+            if (!slow) {
+                // this lane's column
+                float w[UC];
+                float B = 1.f, first = 0.f;
+                int zs = 0, cidx = 0;
+                bool any = false, bad = false;
+                if (ka + lane <= ke) {
+                    const int k = ka + lane;
+                    const float cen = vox(g.d_pix, io, no), bx = vox(g.d_pix, k, nd);
+                    const float x = xdrv ? bx : cen, y = xdrv ? cen : bx;
+                    const SfCol C = sf_col(g, c, s, x, y);
+                    if (C.t3 > TUa && C.t0 < TUb) {
+                        const float f = inv_du * C.lphi * C.mz / g.dv;
+                        float e = trap_cum(TUa, C);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int j = 4 * warp + q;
-                float pa = 0.f, pb = 0.f;
-                if (j < nuT) {
-                    const int f0 = T.cf[b][j], n = T.cn[b][j];
-                    for (int m = 0; m < n; ++m) {
-                        const float w = T.w[b][j][m];
-                        const float *gr = T.gv[b][f0 + m];
-                        pa = fmaf(w, gr[lane + 1] - gr[lane], pa);
-                        pb = fmaf(w, gr[33 + lane] - gr[32 + lane], pb);
+                        for (int q = 0; q < UC; ++q) {
+                            const float t = trap_cum(uedge(g, u0 + q + 1), C);
+                            w[q] = q < nuT ? (t - e) * f : 0.f;
+                            any |= w[q] != 0.f;
+                            e = t;
+                        }
+                        B = kB * (g.DSO - fmaf(c, x, s * y));
+                        const float t = B * vd, tf = floorf(t);
+                        const int fl = (int)tf + (int)ci;
+                        zs = VEC == 4 ? fl & ~3 : fl;
+                        first = (t - tf) + cf + (float)(fl - zs - MID);
+                        const int ze = zs + __float2int_rd(fmaf(B, (float)zn, first)) + MID + 1;
+                        if (ze <= 0 || zs >= g.nz) any = false;
+                        bad = any && (B > NW - 1.0f || ze - zs > BW - NW + 1);
+                        cidx = xdrv ? k * g.ny + io : io * g.ny + k;
                     }
                 }
-                part[2 * q] = pa;
-                part[2 * q + 1] = pb;
-            }
-        } else {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int j = u0 + 4 * warp + q;
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int l = v0 + 32 * hh + lane;
-                    part[2 * q + hh] = (j < g.nu && l < g.nv)
-                        ? sf_cell_line(g, vol, c, s, xdrv, nd, no, io, kA, kB, uedge(g, j),
-                                       uedge(g, j + 1), vedge(g, l), vedge(g, l + 1))
-                        : 0.f;
+                cols = __ballot_sync(0xffffffffu, any);
+                slow = __any_sync(0xffffffffu, bad);
+                if (any) {
+                    *reinterpret_cast<float4 *>(&W.w[lane][0]) = make_float4(w[0], w[1], w[2], w[3]);
+                    *reinterpret_cast<float4 *>(&W.w[lane][4]) = make_float4(w[4], w[5], w[6], w[7]);
+                    W.rec[lane] = make_float4(B, first, __int_as_float(zs), __int_as_float(cidx));
                 }
+                __syncwarp();
+            }
+            if (slow) {
+#pragma unroll
+                for (int q = 0; q < UC; ++q)
+#pragma unroll
+                    for (int m = 0; m < M; ++m) {
+                        const int iv = v0 + 32 * m + lane;
+                        if (q < nuT && iv < g.nv)
+                            (q & 1 ? grp[q / 2][m].y : grp[q / 2][m].x) +=
+                                sf_cell_line(g, vol, c, s, xdrv, nd, no, io, ka, ke, uedge(g, u0 + q),
+                                             uedge(g, u0 + q + 1), vedge(g, iv), vedge(g, iv + 1));
+                    }
+            } else if (!cols) {
+                continue;
+            } else {
+                int win = 0;
+                float2 r[2];
+                float4 rc;
+                unsigned in = 0;
+                auto load = [&](int t) {  // column t's slices that this lane loads, clamped to the volume
+                    rc = W.rec[t];
+                    const int zs = __float_as_int(rc.z);
+                    win = __float2int_rd(fmaf(rc.x, (float)zn, rc.y)) + MID + NW;
+                    const char *p = ptr_at(reinterpret_cast<const char *>(vol), __float_as_int(rc.w), 4u * g.nz);
+                    in = 0;
+                    auto at = [&](int i) {
+                        const int z = zs + min(VEC == 4 ? 4 * lane : lane + 32 * i, (win - 1) & ~(VEC - 1));
+                        const int zc = min(max(z, 0), g.nz - VEC);
+                        in |= (unsigned)(zc == z) << i;
+                        return p + 4 * zc;
+                    };
+                    if (VEC == 4) {
+                        const float4 f = __ldg(reinterpret_cast<const float4 *>(at(0)));
+                        r[0] = make_float2(f.x, f.y);
+                        r[1] = make_float2(f.z, f.w);
+                    } else {
+                        r[0] = make_float2(__ldg(reinterpret_cast<const float *>(at(0))),
+                                           __ldg(reinterpret_cast<const float *>(at(1))));
+                        if (win > 64)
+                            r[1] = make_float2(__ldg(reinterpret_cast<const float *>(at(2))),
+                                               __ldg(reinterpret_cast<const float *>(at(3))));
+                    }
+                };
+                int t = __ffs(cols) - 1, buf = 0;
+                load(t);
+                for (;;) {
+                    float *T = W.T[buf];
+                    buf ^= 1;
+                    // slices outside the volume count as 0
+                    if (VEC == 4) {
+                        if (4 * lane < win)
+                            *reinterpret_cast<float4 *>(T + 4 * lane) =
+                                in ? make_float4(r[0].x, r[0].y, r[1].x, r[1].y) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    } else {
+                        T[lane] = in & 1 ? r[0].x : 0.f;
+                        T[lane + 32] = in & 2 ? r[0].y : 0.f;
+                        if (win > 64) {
+                            T[lane + 64] = in & 4 ? r[1].x : 0.f;
+                            T[lane + 96] = in & 8 ? r[1].y : 0.f;
+                        }
+                    }
+                    __syncwarp();
+                    const float4 cur = rc;
+                    const float4 wa = *reinterpret_cast<const float4 *>(&W.w[t][0]);
+                    const float4 wb = *reinterpret_cast<const float4 *>(&W.w[t][4]);
+                    cols &= cols - 1;
+                    if (cols) {
+                        t = __ffs(cols) - 1;
+                        load(t);
+                    }
+                    // this column's profile at the lane's v cells
+                    float p[M];
+                    bool odd = false;
+#pragma unroll
+                    for (int m = 0; m < M; ++m) {
+                        const float vm = (float)(32 * m + lane);
+                        const float tl = fmaf(cur.x, vm, cur.y), th = fmaf(cur.x, vm + 1.0f, cur.y);
+                        const float tf = floorf(tl);
+                        const float *q = T + min((int)tf + MID, BW - NW);  // v cells past the detector read anything
+                        float a = (fminf(th, tf + 1.0f) - tl) * q[0];
+                        a = fmaf(__saturatef(th - (tf + 1.0f)), q[1], a);
+#pragma unroll
+                        for (int i = 2; i < NW; ++i) {
+                            const float wi = __saturatef(th - (tf + (float)i));
+                            a = fmaf(wi, lds_if(q + i, wi), a);
+                        }
+                        p[m] = a;
+                        odd |= !(fabsf(a) < INFINITY);
+                    }
+                    const float2 w2[UC / 2] = {make_float2(wa.x, wa.y), make_float2(wa.z, wa.w),
+                                               make_float2(wb.x, wb.y), make_float2(wb.z, wb.w)};
+                    if (!__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+                        for (int q = 0; q < UC / 2; ++q)
+#pragma unroll
+                            for (int m = 0; m < M; ++m) grp[q][m] = pk_fma(w2[q], dup(p[m]), grp[q][m]);
+                    } else {  // infinities and NaN only to the cells that the column covers
+#pragma unroll
+                        for (int q = 0; q < UC / 2; ++q)
+#pragma unroll
+                            for (int m = 0; m < M; ++m) {
+                                if (w2[q].x != 0.f) grp[q][m].x = fmaf(w2[q].x, p[m], grp[q][m].x);
+                                if (w2[q].y != 0.f) grp[q][m].y = fmaf(w2[q].y, p[m], grp[q][m].y);
+                            }
+                    }
+                    if (!cols) break;
+                }
+                __syncwarp();  // the table and the row buffers are reused
+            }
+            if (++ngrp == 16) {
+#pragma unroll
+                for (int q = 0; q < UC; ++q)
+#pragma unroll
+                    for (int m = 0; m < M; ++m) {
+                        acc[q * SZ + 32 * m] += q & 1 ? grp[q / 2][m].y : grp[q / 2][m].x;
+                        if (q & 1) grp[q / 2][m] = dup(0.f);
+                    }
+                ngrp = 0;
             }
         }
-#pragma unroll
-        for (int q = 0; q < 8; ++q) grp[q] += part[q];
-        if (++ngrp == 16) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q) { acc[q] += grp[q]; grp[q] = 0.f; }
-            ngrp = 0;
-        }
-        io = nxt;
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int j = u0 + 4 * warp + q;
+    for (int q = 0; q < UC; ++q)
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int l = v0 + 32 * hh + lane;
+        for (int m = 0; m < M; ++m) {
+            const int j = u0 + q, l = v0 + 32 * m + lane;
             if (j < g.nu && l < g.nv) {
                 const float uc = ucen(g, j), vc = vcen(g, l);
                 const float lth = sqrtf(1.f + vc * vc / (uc * uc + g.DSD * g.DSD));
-                sino[((size_t)ia * g.nu + j) * g.nv + l] = (acc[2 * q + hh] + grp[2 * q + hh]) * lth;
+                sino[((size_t)ia * g.nu + j) * g.nv + l] = 
+                    (acc[q * SZ + 32 * m] + (q & 1 ? grp[q / 2][m].y : grp[q / 2][m].x)) * lth;
             }
         }
-    }
+}
+
+template <int VEC, int M>
+int launch_fp(const vg_dd3d_geom *g, const float *vol, const double *trig, float *sino, cudaStream_t st) {
+    constexpr size_t smem = SFW * (sizeof(SfFpWarp) + UC * 32 * M * sizeof(float));
+    int s = cuda_status(cudaFuncSetAttribute(sf3d_fp_kernel<VEC, M>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "sf3d_fp");
+    if (s) return s;
+    dim3 grid(ceil_div(g->nv, 32 * M), ceil_div(g->nu, UC * SFW), g->na);
+    sf3d_fp_kernel<VEC, M><<<grid, 32 * SFW, smem, st>>>(*g, vol, trig, sino);
+    return launch_status("sf3d_fp");
 }
 
 // ---------------------------------------------------------------------------
@@ -434,8 +466,11 @@ __global__ void sf3d_weight(vg_dd3d_geom g, const float *__restrict__ sino, int 
 // Columns over more than 4 u cells, or whose slices reach more cells than the
 // buffer holds, take a per-voxel path.  With too few tiles to fill the GPU the
 // blocks of a cluster share a tile's views; sums meet in rank order.
+//
+// 256^3, 360 views of 512 x 384: 43.0 -> 16.6 ms (62 instructions per 32 voxels and
+// view against 228, bound by issue and the latency of the loads; 2 blocks per SM
+// 18.1 ms).
 constexpr int BT = 8, BKU = 4;
-constexpr int BW = 128, MID = 40;  // cells of a row buffer, and where their count starts
 constexpr int BP_GROUP = 16;
 
 struct SfBpWarp {
@@ -584,10 +619,12 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
                     const int win = __float2int_rd(fmaf(rc.x, (float)zn, rc.y)) + MID + NW;
                     // this lane's cells, clamped to the window and the detector
                     int vo[NV];
+                    unsigned in = 0;
 #pragma unroll
                     for (int i = 0; i < NV; ++i) {
                         const int v = vs + min(VEC == 4 ? 4 * lane : lane + 32 * i, (win - 1) & ~(VEC - 1));
                         vo[i] = 4 * min(max(v, 0), g.nv - VEC);
+                        in |= (unsigned)(vo[i] == 4 * v) << i;
                     }
                     const char *p = VEC == 4 ? q + vo[0] : q;
                     auto load = [&](unsigned jj, float2 (&r)[2]) {
@@ -616,10 +653,19 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
 #pragma unroll
                         for (int i = 0; i < 2; ++i) o[h][i] = pk_fma(dup(w.w), r0[i], o[h][i]);
                     }
-                    if (n == 0) o[h][0] = o[h][1] = dup(0.f);  // nothing from its nearest u cell
+                    // nothing from the nearest u cell of a column beside the detector, and from
+                    // v cells outside it
+                    if (n == 0) in = 0;
+                    if (VEC == 4) {
+                        if (!in) o[h][0] = o[h][1] = dup(0.f);
+                    } else {
+                        if (!(in & 1)) o[h][0].x = 0.f;
+                        if (!(in & 2)) o[h][0].y = 0.f;
+                        if (!(in & 4)) o[h][1].x = 0.f;
+                        if (!(in & 8)) o[h][1].y = 0.f;
+                    }
                     // overlaps of this lane's slices with their cells
                     float over = 0.f;
-                    int qf[M];
 #pragma unroll
                     for (int m = 0; m < M; ++m) {
                         const float zm = (float)(32 * m + lane);
@@ -629,17 +675,9 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
 #pragma unroll
                         for (int t = 1; t < NW; ++t) wv[h][m][t] = __saturatef(th - (tf + (float)t));
                         if (32 * m + lane < zn) over = fmaxf(over, th - tf);
-                        qf[m] = (int)tf + MID;
-                        qi[h][m] = min(qf[m], BW - NW);  // slices past the volume read anything
+                        qi[h][m] = min((int)tf + MID, BW - NW);  // slices past the volume read anything
                     }
                     two[h] = !__any_sync(0xffffffffu, over > 2.0f);
-                    if (vs < 0 || vs + win > g.nv) {
-#pragma unroll
-                        for (int m = 0; m < M; ++m)
-#pragma unroll
-                            for (int t = 0; t < NW; ++t)
-                                if ((unsigned)(qf[m] + vs + t) >= (unsigned)g.nv) wv[h][m][t] = 0.f;
-                    }
                     if (VEC == 4) {
                         if (4 * lane < win)
                             *reinterpret_cast<float4 *>(T[h] + 4 * lane) =
@@ -731,9 +769,8 @@ int check(const vg_dd3d_geom *g) {
     VG_REQUIRE(g->nx > 0 && g->ny > 0 && g->nz > 0 && g->na > 0 && g->nu > 0 && g->nv > 0,
                "sf3d: sizes must be positive");
     VG_REQUIRE(g->na < 65536 && ceil_div(g->nx, BT) < 65536 && ceil_div(g->ny, BT) < 65536 &&
-                   ceil_div(g->nu, SU) < 65536, "sf3d: sizes too large");
-    VG_REQUIRE(g->nx <= SLINES && g->ny <= SLINES, "sf3d: nx and ny at most %d", SLINES);
-    // (nz + 1: the forward projection's z sums index the volume's columns with one extra entry)
+                   ceil_div(g->nu, 32) < 65536, "sf3d: sizes too large");
+    VG_REQUIRE(g->nx <= 2048 && g->ny <= 2048, "sf3d: nx and ny at most 2048");
     VG_REQUIRE((double)g->nx * g->ny * (g->nz + 1) < 2147483648.0, "sf3d: volume above 2^31 voxels");
     VG_REQUIRE(g->du > 0.f && g->dv > 0.f && g->d_pix > 0.f && g->DSO > 0.f && g->DSD > 0.f,
                "sf3d: pitches and distances must be positive");
@@ -759,7 +796,8 @@ size_t bp_ws_bytes(const vg_dd3d_geom *g) {
     return chunk_views(g) * (size_t)g->nu * g->nv * sizeof(float);
 }
 
-// the forward projection's z-prefix array: nx ny (nz + 1) floats
+// kept from when the forward projection formed z sums of the volume's columns:
+// callers size and check their workspace by it
 size_t fp_ws_bytes(const vg_dd3d_geom *g) {
     return (size_t)g->nx * g->ny * (g->nz + 1) * sizeof(float);
 }
@@ -782,14 +820,17 @@ extern "C" int vg_sf3d_fp(const vg_dd3d_geom *g, const float *vol, const double 
                "sf3d_fp: workspace of %zu bytes needed (vg_sf3d_workspace_bytes)", need);
     VG_REQUIRE(((uintptr_t)workspace & 3) == 0, "sf3d_fp: workspace must be 4-byte aligned");
     cudaStream_t s = as_stream(stream);
-    float *zp = static_cast<float *>(workspace);
-    const size_t ncol = (size_t)g->nx * g->ny;
-    sf3d_zprefix<<<ceil_div((long long)ncol * 32, 256), 256, 0, s>>>(*g, vol, zp);
-    st = launch_status("sf3d_zprefix");
-    if (st) return st;
-    dim3 grid(ceil_div(g->nv, SV), ceil_div(g->nu, SU), g->na);
-    sf3d_fp_kernel<<<grid, 256, 0, s>>>(*g, vol, zp, trig, sino);
-    return launch_status("sf3d_fp");
+    // 96 or 64 v cells per warp while the slices under them fit a row buffer, by the
+    // smallest magnification in the volume; 96 unless the detector's last tile is
+    // emptier for it; 16-byte loads where columns are aligned
+    const double r = 0.5 * hypot((double)g->nx, (double)g->ny) * g->d_pix;
+    const double bmax = (g->DSO + r) / g->DSD * g->dv / g->d_pix;
+    const bool vec = g->nz % 4 == 0 && ((uintptr_t)vol & 15) == 0;
+    if (g->nv > 32 && 96.0 * bmax + 9.0 <= BW && 96 * ceil_div(g->nv, 96) <= 1.15 * 64 * ceil_div(g->nv, 64))
+        return vec ? launch_fp<4, 3>(g, vol, trig, sino, s) : launch_fp<1, 3>(g, vol, trig, sino, s);
+    if (g->nv > 32 && 64.0 * bmax + 9.0 <= BW)
+        return vec ? launch_fp<4, 2>(g, vol, trig, sino, s) : launch_fp<1, 2>(g, vol, trig, sino, s);
+    return vec ? launch_fp<4, 1>(g, vol, trig, sino, s) : launch_fp<1, 1>(g, vol, trig, sino, s);
 }
 
 extern "C" int vg_sf3d_bp(const vg_dd3d_geom *g, const float *sino, const double *trig, float *vol,
