@@ -191,6 +191,11 @@ int vg_dd2d_fp_default_variant(const vg_dd2d_geom *g);
 int vg_dd2d_fp(const vg_dd2d_geom *g, const float *img, const float *imgT,
                const double *trig, float *sino, void *stream);
 
+/* The same from the image alone: imgT (ny, nx) is scratch, which the call fills
+ * with the transpose first. */
+int vg_dd2d_fp_plain(const vg_dd2d_geom *g, const float *img, float *imgT,
+                     const double *trig, float *sino, void *stream);
+
 /* Bytes of device workspace vg_dd2d_bp and vg_dd2d_sirt_iter need for this
  * geometry (per-view running integrals of the sinogram rows and line
  * scales); 0 for an invalid geometry. */

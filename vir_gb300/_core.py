@@ -16,12 +16,15 @@ import threading
 import numpy as np
 import torch
 
+from . import _lib
 from ._lib import VirGpuError, call, load  # noqa: F401
 
 _F32 = torch.float32
 
 
 def require_cuda():
+    if torch.cuda.is_initialized() and _lib._lib is not None:
+        return  # a context and the library are there (the full check costs 4 us a call)
     if not torch.cuda.is_available():
         raise VirGpuError("device", -1, "vir_gb300 needs a CUDA device; none is visible")
     load()
@@ -43,6 +46,8 @@ def to_device(a, dev=None, dtype=_F32) -> torch.Tensor:
     require_cuda()
     dev = dev or device_of(a)
     if is_torch(a):
+        if a.dtype is dtype and not a.requires_grad and a.device == dev and a.is_contiguous():
+            return a
         t = a.detach().to(device=dev, dtype=dtype)
     else:
         t = torch.from_numpy(np.ascontiguousarray(np.asarray(a), dtype=np.dtype(str(dtype).split(".")[-1])))
@@ -63,11 +68,14 @@ def ptr(t: torch.Tensor) -> int:
 
 
 def stream(dev=None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    if dev is None or dev.index is None:
+        return ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    # the same handle without building a Stream object (5 us)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(dev.index))
 
 
 def empty(shape, dev, dtype=_F32) -> torch.Tensor:
-    return torch.empty(tuple(int(s) for s in shape), dtype=dtype, device=dev)
+    return torch.empty([int(s) for s in shape], dtype=dtype, device=dev)
 
 
 def host_angles(a) -> np.ndarray:
@@ -89,7 +97,7 @@ class _TrigCache:
     def get(self, angles, cast=None, dev=None) -> torch.Tensor:
         a = host_angles(angles)
         if cast is not None:
-            a = a.astype(cast)
+            a = a.astype(cast, copy=False)
         dev = dev or torch.device("cuda", torch.cuda.current_device())
         key = (a.dtype.str, a.shape, a.tobytes(), str(dev))
         with self._lock:
@@ -113,4 +121,7 @@ trig_cache = _TrigCache()
 
 def f32(v) -> float:
     """Round a scalar to float32 as vir's as_float32 does (dd.py:29-36)."""
-    return float(np.float32(v))
+    try:
+        return ctypes.c_float(v).value  # the same rounding as np.float32, a third of its time
+    except TypeError:
+        return float(np.float32(v))

@@ -105,6 +105,7 @@ _PROTOS = {
     "vg_list_fp": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p],
     "vg_list_bp": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int,
                    c_void_p, c_size_t, c_void_p],
+    "vg_dd2d_fp_plain": [ctypes.POINTER(DD2DGeom), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     "vg_dd2d_fp": [ctypes.POINTER(DD2DGeom), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     "vg_dd2d_bp": [ctypes.POINTER(DD2DGeom), c_void_p, c_void_p, c_void_p, c_void_p, c_size_t,
                    c_void_p],
@@ -264,4 +265,4 @@ def dd2d_workspace(g, dev):
         raise VirGpuError("vg_dd2d_workspace_bytes", 1, L.vg_last_error().decode(errors="replace"))
     t = torch.empty(n + 256, dtype=torch.uint8, device=dev)
     off = (-t.data_ptr()) % 256
-    return t[off:off + n]
+    return t[off:off + n] if off else t

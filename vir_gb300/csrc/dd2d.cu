@@ -1240,6 +1240,34 @@ extern "C" int vg_dd2d_fp(const vg_dd2d_geom *g, const float *img, const float *
     return launch_fp(g, img, imgT, trig, sino, 0, nullptr, nullptr, as_stream(stream));
 }
 
+namespace {
+// out (cols, rows) = in (rows, cols) transposed, 32 x 32 tiles
+__global__ void __launch_bounds__(256) transpose2d(const float *__restrict__ in, int rows, int cols,
+                                                   float *__restrict__ out) {
+    __shared__ float tile[32][33];
+    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+    for (int q = threadIdx.y; q < 32; q += 8)
+        if (r0 + q < rows && c0 + threadIdx.x < cols)
+            tile[q][threadIdx.x] = __ldg(in + (size_t)(r0 + q) * cols + c0 + threadIdx.x);
+    __syncthreads();
+    for (int q = threadIdx.y; q < 32; q += 8)
+        if (c0 + q < cols && r0 + threadIdx.x < rows)
+            out[(size_t)(c0 + q) * rows + r0 + threadIdx.x] = tile[threadIdx.x][q];
+}
+}  // namespace
+
+extern "C" int vg_dd2d_fp_plain(const vg_dd2d_geom *g, const float *img, float *imgT, const double *trig,
+                                float *sino, void *stream) {
+    int st = check_geom(g);
+    if (st) return st;
+    VG_REQUIRE(img && imgT && trig && sino, "dd2d_fp_plain: null pointer");
+    dim3 grid(ceil_div(g->ny, 32), ceil_div(g->nx, 32));
+    transpose2d<<<grid, dim3(32, 8), 0, as_stream(stream)>>>(img, g->nx, g->ny, imgT);
+    st = launch_status("dd2d_fp_plain: transpose");
+    if (st) return st;
+    return launch_fp(g, img, imgT, trig, sino, 0, nullptr, nullptr, as_stream(stream));
+}
+
 extern "C" int vg_dd2d_fp_variants(void) { return FP_NVARIANTS; }
 
 extern "C" int vg_dd2d_fp_default_variant(const vg_dd2d_geom *g) {

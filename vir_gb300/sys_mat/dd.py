@@ -57,9 +57,9 @@ def _fp(img, ang_arr, nu, du, su, d_pix, DSO, DSD, fan):
     trig = _core.trig_cache.get(ang_arr, np.float32, dev)
     na = trig.numel() // 2
     g = _geom(x.shape[0], x.shape[1], na, nu, du, su, d_pix, DSO, DSD, fan)
-    xT = x.t().contiguous()
+    xT = _core.empty((x.shape[1], x.shape[0]), dev)
     sino = _core.empty((na, nu), dev)
-    call("vg_dd2d_fp", ctypes.byref(g), _core.ptr(x), _core.ptr(xT), _core.ptr(trig),
+    call("vg_dd2d_fp_plain", ctypes.byref(g), _core.ptr(x), _core.ptr(xT), _core.ptr(trig),
          _core.ptr(sino), _core.stream(dev))
     return _core.to_host_like(sino, img)
 
