@@ -40,25 +40,14 @@ __device__ __forceinline__ double div_pix(const SidGeom &g, double v) {
 // correctly rounded quotient (Markstein's theorem; Muller et al., Handbook of
 // Floating-Point Arithmetic, division with a fused multiply-add).  Three FP64
 // operations per quotient once y is known; finite, normal operands only.
-#ifndef VG_SID_RCP
-#define VG_SID_RCP 1
-#endif
 __device__ __forceinline__ double div_by(double a, double b, double y) {
-#if VG_SID_RCP
     const double q0 = __dmul_rn(a, y);
     const double r = __fma_rn(-b, q0, a);
     return __fma_rn(r, y, q0);
-#else
-    return d_div(a, b);
-#endif
 }
 
 __device__ __forceinline__ double rcp_of(double b) {
-#if VG_SID_RCP
     return b != 0.0 ? __drcp_rn(b) : 0.0;
-#else
-    return 0.0;
-#endif
 }
 
 struct Ray {
@@ -67,31 +56,31 @@ struct Ray {
     bool valid;
 };
 
-__device__ __forceinline__ Ray ray_setup(const SidGeom &g, int k, double dx, double dy) {
+// rdx, rdy: RN(1 / dx), RN(1 / dy) of the view (rcp_of).  The plane met first
+// along an axis is the first or the last by the direction's sign, which is the
+// lesser of the two quotients because rounding keeps their order.
+__device__ __forceinline__ Ray ray_setup(const SidGeom &g, int k, double dx, double dy, double rdx,
+                                         double rdy) {
     Ray r;
     double det = d_mul(g.d_det, d_add((double)k - (double)g.n_dets * 0.5, 0.5));
     r.x0 = d_mul(det, -dy);
     r.y0 = d_mul(det, dx);
-    r.rdx = rcp_of(dx);
-    r.rdy = rcp_of(dy);
+    r.rdx = rdx;
+    r.rdy = rdy;
     double tx0 = -INFINITY, txn = INFINITY, ty0 = -INFINITY, tyn = INFINITY;
-    if (dx != 0.0) { tx0 = div_by(d_sub(g.xb0, r.x0), dx, r.rdx); txn = div_by(d_sub(g.xbn, r.x0), dx, r.rdx); }
-    if (dy != 0.0) { ty0 = div_by(d_sub(g.yb0, r.y0), dy, r.rdy); tyn = div_by(d_sub(g.ybn, r.y0), dy, r.rdy); }
-    r.t0 = fmax(fmin(tx0, txn), fmin(ty0, tyn));
-    r.t1 = fmin(fmax(tx0, txn), fmax(ty0, tyn));
+    const bool px = dx > 0.0, py = dy > 0.0;
+    if (dx != 0.0) {
+        tx0 = div_by(d_sub(px ? g.xb0 : g.xbn, r.x0), dx, rdx);
+        txn = div_by(d_sub(px ? g.xbn : g.xb0, r.x0), dx, rdx);
+    }
+    if (dy != 0.0) {
+        ty0 = div_by(d_sub(py ? g.yb0 : g.ybn, r.y0), dy, rdy);
+        tyn = div_by(d_sub(py ? g.ybn : g.yb0, r.y0), dy, rdy);
+    }
+    r.t0 = fmax(tx0, ty0);
+    r.t1 = fmin(txn, tyn);
     r.valid = !(r.t1 <= r.t0 || isinf(r.t0) || isinf(r.t1));
     return r;
-}
-
-// Crossing parameter of the j-th plane in traversal order (t non-decreasing
-// in j): index i = j when the direction component is positive, n - j else.
-// The plane position is edge(d_pix, i, n), read from `et` (a table of the
-// same values) when given.
-__device__ __forceinline__ double cross_t(double d_pix, int n, int j, bool pos, double o, double d,
-                                          double rd, const double *et = nullptr) {
-    int i = pos ? j : n - j;
-    const double e = et ? et[i] : edge(d_pix, i, n);
-    return div_by(d_sub(e, o), d, rd);
 }
 
 // The crossings' comparisons run on integers: ord64 maps doubles (no NaN)
@@ -103,28 +92,72 @@ __device__ __forceinline__ long long ord64(double x) {
     return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
 }
 
-// First traversal index whose crossing is >= t0 (n + 1 when none).
-__device__ int first_crossing(double d_pix, int n, bool pos, double o, double d, double rd,
-                              double t0, double b0, const double *et = nullptr) {
-    double p = d_add(o, d_mul(t0, d));
-    double fi = floor((p - b0) / d_pix);
-    int j = (int)fmin(fmax(pos ? fi : (double)n - fi, 0.0), (double)(n + 1));
-    // settle on the exact boundary (a handful of steps at most)
-    for (int it = 0; it < 4 && j > 0 && cross_t(d_pix, n, j - 1, pos, o, d, rd, et) >= t0; ++it) --j;
-    while (j > 0 && cross_t(d_pix, n, j - 1, pos, o, d, rd, et) >= t0) --j;
-    while (j <= n && cross_t(d_pix, n, j, pos, o, d, rd, et) < t0) ++j;
-    return j;
+// One axis of a ray's walk: the plane `i` of its next crossing (stepped by s),
+// that crossing's parameter t and its ord64 image o (DONE past the last plane
+// and on an axis the ray does not move along).
+constexpr long long DONE = 0x7fffffffffffffffLL;
+struct Axis {
+    double o0, d, rd;  // origin, direction, RN(1 / d)
+    int n, s, i;
+    double t;
+    long long o;
+};
+
+// Crossing of plane i.  The plane position is edge(d_pix, i, n), read from
+// `et` (a table of the same values) when given.
+__device__ __forceinline__ double cross_at(const Axis &a, double d_pix, int i, const double *et) {
+    return div_by(d_sub(et ? et[i] : edge(d_pix, i, a.n), a.o0), a.d, a.rd);
 }
 
-// Last traversal index whose crossing is <= t1 (-1 when none).
-__device__ int last_crossing(double d_pix, int n, bool pos, double o, double d, double rd,
-                             double t1, double b0, const double *et) {
-    double p = d_add(o, d_mul(t1, d));
-    double fi = floor((p - b0) / d_pix);
-    int j = (int)fmin(fmax(pos ? fi : (double)n - fi, -1.0), (double)n);
-    while (j >= 0 && cross_t(d_pix, n, j, pos, o, d, rd, et) > t1) --j;
-    while (j < n && cross_t(d_pix, n, j + 1, pos, o, d, rd, et) <= t1) ++j;
-    return j;
+// The first crossing at or after tb (crossings are non-decreasing along the
+// walk).  The plane guessed from tb is settled against the crossings
+// themselves, so the guess's rounding does not show in the result.
+__device__ __forceinline__ void axis_start(Axis &a, const SidGeom &g, double o0, double d, double rd,
+                                           int n, double tb, const double *et) {
+    a.o0 = o0; a.d = d; a.rd = rd; a.n = n;
+    a.s = __double2hiint(d) >= 0 ? 1 : -1;  // read again at each step: not an FP64 compare
+    a.i = 0;
+    a.t = 0.0;
+    a.o = DONE;
+    if (d == 0.0) return;
+    const long long ob = ord64(tb);
+    // planes below the point at tb; the first one ahead of it
+    const int below = __double2int_rd(fma(fma(tb, d, o0), g.inv_dpix, 0.5 * n));
+    int i = max(-1, min(n + 1, a.s > 0 ? min(below, n) + 1 : below));
+    if (a.s > 0 ? i < 0 : i > n) i -= a.s;  // the walk's first plane at the earliest
+    if ((unsigned)i <= (unsigned)n) {
+        a.t = cross_at(a, g.d_pix, i, et);
+        a.o = ord64(a.t);
+    }
+    if (a.o < ob) {
+        do {
+            i += a.s;
+            a.o = DONE;
+            if ((unsigned)i > (unsigned)n) break;
+            a.t = cross_at(a, g.d_pix, i, et);
+            a.o = ord64(a.t);
+        } while (a.o < ob);
+    } else {
+        while ((unsigned)(i - a.s) <= (unsigned)n) {
+            const double t = cross_at(a, g.d_pix, i - a.s, et);
+            const long long o = ord64(t);
+            if (o < ob) break;
+            i -= a.s;
+            a.t = t;
+            a.o = o;
+        }
+    }
+    a.i = i;
+}
+
+// (float)h for h >= 2^-126, rounded to nearest even on the integer pipe (the
+// conversion instruction runs at the FP64 rate).
+__device__ __forceinline__ float to_f32(double h) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(h);
+    const unsigned long long u = b + 0x0fffffffULL + ((b >> 29) & 1);
+    return (unsigned)(u >> 52) <= 1150u
+               ? __uint_as_float((unsigned)(u >> 29) - 0xc0000000u)  // exponent - (1023 - 127)
+               : INFINITY;
 }
 
 // TRACE: instead of the line integral, record per ray the number of
@@ -157,161 +190,141 @@ struct Slots {
 // or after tau_part, as the single walk starts from those at or after t0, so
 // the parts together visit the single walk's segments, each once.  MODE 0
 // adds the parts' sums in part order; the trace needs one walk (P = 1).
-#ifndef VG_SID_TAB
-#define VG_SID_TAB 1
-#endif
-#ifndef VG_SID_TAB_MAX
-#define VG_SID_TAB_MAX 2048  // plane positions held in shared memory (16 KB)
-#endif
-#ifndef VG_SID_TRAV
-#define VG_SID_TRAV 1
-#endif
-#ifndef VG_SID_PARTS
-#define VG_SID_PARTS 8
-#endif
+//
+// Bound by the FP64 pipe, which takes a warp instruction only every 16 cycles
+// of an SM whatever the number of its active lanes, so the walk's step counts
+// FP64 instructions a warp issues: five, the quotient's four (shared by the
+// two axes) and the length's difference.  Comparisons, directions, the cell
+// and the length's rounding to FP32 are integer work.  256^2, 180 views, 367
+// bins: 0.94 -> 0.30 ms forward and 0.81 -> 0.31 ms scatter against separate
+// steps per axis (four more FP64 instructions), cells set from the midpoint's
+// floors, FP64 compares, conversions and a division in each part's start.
+// 8 parts: 4 leave the SMs' last wave uneven (0.80 ms the pair against 0.75),
+// 16 pay the start twice as often (0.90).  256 threads share a block's tables
+// (0.75 ms the pair; 128: 0.76).
+constexpr int SID_TAB_MAX = 2048;  // plane positions held in shared memory (16 KB)
+constexpr int SID_PARTS = 8;
+constexpr int SID_BLOCK = 256;
 template <int MODE, int P>
-__global__ void
+__global__ void __launch_bounds__(SID_BLOCK)
 siddon2d_fp_kernel(SidGeom g, const float *__restrict__ img, const double *__restrict__ trig,
                    int na, float *__restrict__ sino, Trace tr, Slots sl) {
     static_assert(P == 1 || (MODE != 1 && 32 % P == 0), "parts split rays in MODE 0 and 2");
     constexpr bool TRACE = MODE == 1;
-    // the plane positions of both axes, once per block (the same FP64 values
-    // edge() computes), when they fit
-    __shared__ double etab[VG_SID_TAB_MAX];
-    const bool tab = VG_SID_TAB && g.nx + g.ny + 2 <= VG_SID_TAB_MAX;
+    // the plane positions of both axes (the same FP64 values edge() computes),
+    // when they fit, and the view's reciprocals, once per block
+    __shared__ double etab[SID_TAB_MAX];
+    __shared__ double srcp[2];
+    int ia = blockIdx.y + sl.ia0;
+    const bool tab = g.nx + g.ny + 2 <= SID_TAB_MAX;
+    const double dx = trig[2 * ia], dy = trig[2 * ia + 1];
     if (tab) {
         for (int i = threadIdx.x; i <= g.nx; i += blockDim.x) etab[i] = edge(g.d_pix, i, g.nx);
         for (int i = threadIdx.x; i <= g.ny; i += blockDim.x) etab[g.nx + 1 + i] = edge(g.d_pix, i, g.ny);
     }
+    if (threadIdx.x < 2) srcp[threadIdx.x] = rcp_of(threadIdx.x ? dy : dx);
     __syncthreads();
     const double *etx = tab ? etab : nullptr, *ety = tab ? etab + g.nx + 1 : nullptr;
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     const int k = gid / P, part = gid % P;
-    int ia = blockIdx.y + sl.ia0;
-    if (k >= g.n_dets || ia >= na) return;  // whole groups of P lanes
+    if (k >= g.n_dets) return;  // whole groups of P lanes
     const float yv = MODE == 2 ? __ldg(sl.y + (size_t)ia * g.n_dets + k) : 0.f;
     float *slot = MODE == 2 ? sl.buf + (size_t)blockIdx.y * g.nx * g.ny * sl.S + k % sl.S : nullptr;
-    double dx = trig[2 * ia], dy = trig[2 * ia + 1];
-    Ray r = ray_setup(g, k, dx, dy);
+    Ray r = ray_setup(g, k, dx, dy, srcp[0], srcp[1]);
     Kahan acc;
     int tcount = 0;
     unsigned long long thash = 0xCBF29CE484222325ull;
     double tlen = 0.0;
     if (r.valid) {
-        const double INF = INFINITY;
         // this part's range [tbeg, tend) of segment starts
         const double span = d_sub(r.t1, r.t0);
         const double tbeg = part == 0 ? r.t0 : d_add(r.t0, d_mul(span, (double)part / P));
-        const double tend = part == P - 1 ? INF : d_add(r.t0, d_mul(span, (double)(part + 1) / P));
-        bool px = dx > 0.0, py = dy > 0.0;
-        // crossings jx..jx_end of the x planes (and y) lie in [tbeg, t1]
-        int jx = 0, jy = 0, jx_end = -1, jy_end = -1;
-        double tx = 0.0, ty = 0.0;
-        long long ox = 0, oy = 0;  // ord64 of tx, ty
-        if (dx != 0.0) {
-            jx = first_crossing(g.d_pix, g.nx, px, r.x0, dx, r.rdx, tbeg, g.xb0, etx);
-            jx_end = last_crossing(g.d_pix, g.nx, px, r.x0, dx, r.rdx, r.t1, g.xb0, etx);
-            if (jx <= jx_end) {
-                tx = cross_t(g.d_pix, g.nx, jx, px, r.x0, dx, r.rdx, etx);
-                ox = ord64(tx);
-            }
-        }
-        if (dy != 0.0) {
-            jy = first_crossing(g.d_pix, g.ny, py, r.y0, dy, r.rdy, tbeg, g.yb0, ety);
-            jy_end = last_crossing(g.d_pix, g.ny, py, r.y0, dy, r.rdy, r.t1, g.yb0, ety);
-            if (jy <= jy_end) {
-                ty = cross_t(g.d_pix, g.ny, jy, py, r.y0, dy, r.rdy, ety);
-                oy = ord64(ty);
-            }
-        }
-        bool xa = jx <= jx_end, ya = jy <= jy_end;  // axes with crossings left
-        bool have_prev = false;
+        const long long oend =
+            part == P - 1 ? DONE : ord64(d_add(r.t0, d_mul(span, (double)(part + 1) / P)));
+        const long long o1 = ord64(r.t1);  // no crossing after t1 belongs to the ray
+        Axis ax, ay;
+        axis_start(ax, g, r.x0, dx, r.rdx, g.nx, tbeg, etx);
+        axis_start(ay, g, r.y0, dy, r.rdy, g.ny, tbeg, ety);
         double tprev = 0.0;
-        long long oprev = 0;
-        const long long oend = ord64(tend);
+        long long oprev = DONE;  // no crossing yet: nothing exceeds it
         // A segment's voxel is vir's floor of its midpoint.  The midpoint lies at
         // least h |d| / 2 (h = tn - tprev) from the cell's boundaries along each
         // axis (less the crossings' own rounding), and its computed coordinates
         // are within a few FP64 ulps of L = the ray's largest coordinate or
         // parameter magnitude, so when h |dx| and h |dy| both exceed 1e-9 L the
-        // floors are the cell the walk is in: the walk's cell (cx, cy), set from
-        // the floors of the first such segment and stepped at every crossing,
-        // is used; shorter segments (and rays nearly along an axis) take the
-        // floors.
+        // floors are the cell between the planes the walk is in: the one just
+        // before the next plane of each axis (cell = plane - 1 along a
+        // positive direction, else plane).  Shorter segments (and rays nearly along an
+        // axis) take the floors; along an axis the ray does not move on, the
+        // cell is the origin's.
         const double L = 1.0 + fabs(r.t0) + fabs(r.t1) + fabs(r.x0) + fabs(r.y0) + fabs(g.xb0) +
                          fabs(g.yb0);
-        const double thr = VG_SID_TRAV ? 1e-9 * L * fmax(fabs(r.rdx), fabs(r.rdy)) : INF;
-        int cx = 0, cy = 0;
-        bool walk_cell = false;
-        const int sx = px ? 1 : -1, sy = py ? 1 : -1;
+        const long long thr = __double_as_longlong(1e-9 * L * fmax(fabs(r.rdx), fabs(r.rdy)));
+        if (dx == 0.0) ax.i = __double2int_rd(div_pix(g, d_sub(r.x0, g.xb0))) + (ax.s > 0);
+        if (dy == 0.0) ay.i = __double2int_rd(div_pix(g, d_sub(r.y0, g.yb0))) + (ay.s > 0);
+        // Both axes advance through the same instructions, on operands chosen
+        // by which crossing is the earlier: the lanes of a warp differ in it at
+        // nearly every step, and each FP64 instruction that only some lanes
+        // take costs as much as one that all take.
         // bounded: every step consumes one of nx + ny + 2 crossings
         for (int step = 0; step < g.nx + g.ny + 4; ++step) {
-            if (!xa && !ya) break;
             // the earlier crossing; ties take the x plane first
-            const bool xcross = xa && (!ya || ox <= oy);
-            double tn;
-            long long on;
-            if (xcross) {
-                tn = tx;
-                on = ox;
-                ++jx;
-                xa = jx <= jx_end;
-                if (xa) {
-                    tx = cross_t(g.d_pix, g.nx, jx, px, r.x0, dx, r.rdx, etx);
-                    ox = ord64(tx);
-                }
-            } else {
-                tn = ty;
-                on = oy;
-                ++jy;
-                ya = jy <= jy_end;
-                if (ya) {
-                    ty = cross_t(g.d_pix, g.ny, jy, py, r.y0, dy, r.rdy, ety);
-                    oy = ord64(ty);
-                }
-            }
-            if (have_prev && on > oprev) {
-                const double h = d_sub(tn, tprev);
+            const bool xc = ax.o <= ay.o;
+            const long long on = xc ? ax.o : ay.o;
+            if (on > o1) break;
+            const double tn = xc ? ax.t : ay.t;
+            if (on > oprev) {
+                const double h = d_sub(tn, tprev);  // positive
                 int ix, iy;
-                if (walk_cell && h > thr) {
-                    ix = cx;
-                    iy = cy;
+                float w;
+                if (__double_as_longlong(h) > thr) {  // thr >= 1e-9
+                    ix = ax.i - (ax.s > 0);
+                    iy = ay.i - (ay.s > 0);
+                    w = to_f32(h);
                 } else {
+                    w = (float)h;
                     double m = d_mul(0.5, d_add(tprev, tn));
                     double fx = floor(div_pix(g, d_sub(d_add(r.x0, d_mul(m, dx)), g.xb0)));
                     double fy = floor(div_pix(g, d_sub(d_add(r.y0, d_mul(m, dy)), g.yb0)));
                     // outside the grid by more than the int range: no voxel
                     ix = fx >= 0.0 && fx < g.nx ? (int)fx : -1;
                     iy = fy >= 0.0 && fy < g.ny ? (int)fy : -1;
-                    if (!walk_cell && h > thr) {
-                        walk_cell = true;
-                        cx = (int)fmax(fmin(fx, 1e9), -1e9);
-                        cy = (int)fmax(fmin(fy, 1e9), -1e9);
-                    }
                 }
-                if (ix >= 0 && ix < g.nx && iy >= 0 && iy < g.ny) {
+                if ((unsigned)ix < (unsigned)g.nx && (unsigned)iy < (unsigned)g.ny) {
                     size_t pix = (size_t)ix * g.ny + iy;
                     if (TRACE) {
                         ++tcount;
                         thash = trace_mix(thash, pix);
                         tlen = d_add(tlen, h);
                     } else if (MODE == 2) {
-                        slot[pix * sl.S] += __fmul_rn(yv, (float)h);
+                        slot[pix * sl.S] += __fmul_rn(yv, w);
                     } else {
-                        float w = (float)h;
                         acc.add(__fmul_rn(__ldg(img + pix), w));
                     }
                 }
             }
-            // the crossing moves the walk into the next cell along its axis
-            if (walk_cell) {
-                if (xcross) cx += sx;
-                else cy += sy;
-            }
             tprev = tn;
             oprev = on;
-            have_prev = true;
-            if (P > 1 && oprev >= oend) break;  // the next segment starts in the next part
+            if (P > 1 && on >= oend) break;  // the next segment starts in the next part
+            // the chosen axis's next crossing
+            const int i = xc ? ax.i + ax.s : ay.i + ay.s;
+            const int n = xc ? g.nx : g.ny;
+            double t = 0.0;
+            long long o = DONE;
+            if ((unsigned)i <= (unsigned)n) {
+                const double e = tab ? etab[xc ? i : g.nx + 1 + i] : edge(g.d_pix, i, n);
+                t = div_by(d_sub(e, xc ? r.x0 : r.y0), xc ? dx : dy, xc ? r.rdx : r.rdy);
+                o = ord64(t);
+            }
+            if (xc) {
+                ax.i = i;
+                ax.t = t;
+                ax.o = o;
+            } else {
+                ay.i = i;
+                ay.t = t;
+                ay.o = o;
+            }
         }
     }
     if (MODE == 0 && P > 1) {
@@ -400,13 +413,14 @@ siddon2d_bp_kernel(SidGeom g, const float *__restrict__ sino, const double *__re
     Kahan acc;
     for (int ia = 0; ia < na; ++ia) {
         double dx = __ldg(trig + 2 * ia), dy = __ldg(trig + 2 * ia + 1);
+        const double rdx = rcp_of(dx), rdy = rcp_of(dy);
         float fdx = (float)dx, fdy = (float)dy;
         float uc = -fdy * xc + fdx * yc;
         float hw = half * (fabsf(fdx) + fabsf(fdy)) + 1e-3f * (float)g.d_det + 1e-5f * fabsf(uc);
         int k_lo = max(0, (int)ceilf((uc - hw) * inv_det + koff));
         int k_hi = min(g.n_dets - 1, (int)floorf((uc + hw) * inv_det + koff));
         for (int k = k_lo; k <= k_hi; ++k) {
-            Ray r = ray_setup(g, k, dx, dy);
+            Ray r = ray_setup(g, k, dx, dy, rdx, rdy);
             if (!r.valid) continue;
             double tx[4], ty[4], t[8];
             int nx_ = window_crossings(g.d_pix, g.nx, ix - 1, r.x0, dx, r.rdx, r.t0, r.t1, tx);
@@ -457,8 +471,8 @@ extern "C" int vg_siddon2d_fp(const float *img, int nx, int ny, const double *tr
     if (st) return st;
     VG_REQUIRE(na > 0 && na < 65536, "siddon2d_fp: na out of range");
     VG_REQUIRE(img && trig && sino, "siddon2d_fp: null pointer");
-    dim3 grid(ceil_div((long long)n_dets * VG_SID_PARTS, 128), na);
-    siddon2d_fp_kernel<0, VG_SID_PARTS><<<grid, 128, 0, as_stream(stream)>>>(g, img, trig, na, sino, Trace{},
+    dim3 grid(ceil_div((long long)n_dets * SID_PARTS, SID_BLOCK), na);
+    siddon2d_fp_kernel<0, SID_PARTS><<<grid, SID_BLOCK, 0, as_stream(stream)>>>(g, img, trig, na, sino, Trace{},
                                                               Slots{nullptr, nullptr, 1, 0});
     return launch_status("siddon2d_fp");
 }
@@ -549,8 +563,8 @@ extern "C" int vg_siddon2d_bp_scatter(const float *sino, int na, int n_dets, con
         const int nv = na - ia0 < nvc ? na - ia0 : nvc;
         cudaError_t e = cudaMemsetAsync(buf, 0, (size_t)nv * per_view, s);
         if (e != cudaSuccess) return cuda_status(e, "siddon2d_bp_scatter: clear");
-        dim3 grid(ceil_div((long long)n_dets * VG_SID_PARTS, 128), nv);
-        siddon2d_fp_kernel<2, VG_SID_PARTS><<<grid, 128, 0, s>>>(g, nullptr, trig, na, nullptr, Trace{},
+        dim3 grid(ceil_div((long long)n_dets * SID_PARTS, SID_BLOCK), nv);
+        siddon2d_fp_kernel<2, SID_PARTS><<<grid, SID_BLOCK, 0, s>>>(g, nullptr, trig, na, nullptr, Trace{},
                                                      Slots{sino, buf, S, ia0});
         st = launch_status("siddon2d_bp_scatter");
         if (st) return st;
