@@ -78,6 +78,9 @@ __device__ __forceinline__ float2 pk_add_rd(float2 a, float2 b) {
     asm("add.rm.f32x2 %0, %1, %2;" : "=l"(pk_bits(d)) : "l"(pk_bits(a)), "l"(pk_bits(b)));
     return d;
 }
+__device__ __forceinline__ float2 pk_sub(float2 a, float2 b) {  // a - b: -b is exact
+    return pk_fma(b, make_float2(-1.f, -1.f), a);
+}
 __device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
 
 // 1 / d to about half an ulp: the hardware's estimate and one Newton step.
