@@ -76,3 +76,52 @@ def test_taps_nan_stays_near(vg):
     near = torch.nn.functional.max_pool1d((fp(hit) != 0).float()[:, None], 5, 1, 2)[:, 0] > 0
     x[17, 21] = float("nan")
     assert not bool((torch.isnan(fp(x)) & ~near).any())
+
+
+# shape, nu, na (first view at 45 degrees), du, d_pix, DSO, DSD, tolerance.  The share to
+# first order in the bin's change of width (du <= 3e-3 of the source's distance from the
+# detector's end).  "scan" and "fine": bins of 0.67 and 0.17 pixel seen from far, positions
+# within 64 pixels: three roundings of 64 * 2^-24 pixel on steps of at most 1, averaged over
+# 64 lines of independent rounding: 1.5e-6 of a value of half the lines; 1e-5 has six times that.
+# "dot": the source within half a pixel of the corner of a 2 x 2 image, where the share's
+# first order would turn at the next pixel edge; bins down to 4e-4 pixel, so three roundings
+# of 2 * 2^-24 pixel are 9e-4 of a step: 2e-3.
+FIRST_ORDER = {
+    "scan": ((64, 61), 131, 24, 1.2, 0.9, 500.0, 1000.0, 1e-5),
+    "fine": ((64, 64), 400, 16, 0.3, 0.9, 500.0, 1000.0, 1e-5),
+    "dot": ((2, 2), 1600, 8, 0.0012, 1.0, 1.45, 2.2, 2e-3),
+}
+
+
+@pytest.mark.parametrize("name", sorted(FIRST_ORDER))
+def test_taps_first_order_vs_oracle(vg, orc, name):
+    from vir_gb300 import _lib
+    from vir_gb300.sys_mat import dd
+    shape, nu, na, du, d, DSO, DSD, tol = FIRST_ORDER[name]
+    g = _lib.DD2DGeom(*shape, na, nu, du, 0.0, d, DSO, DSD, 1)
+    L = _lib.load()
+    assert L.vg_dd2d_fp_default_variant(ctypes.byref(g)) == L.vg_dd2d_fp_variants()
+    assert du <= 3e-3 * (DSD - 0.5 * nu * du)
+    img = np.random.default_rng(37).random(shape).astype(np.float32)
+    angs = np.pi / 4 + np.linspace(0, 2 * np.pi, na, endpoint=False)
+    f = lambda v: float(np.float32(v))
+    got = dd.dd_fp_fan_2d(img, angs, nu, DSO, DSD, du=du, d_pix=d)
+    ref = orc.dd_fp_fan_2d(img, angs, nu, f(DSO), f(DSD), du=f(du), d_pix=f(d))
+    assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n,nu,du,DSO,DSD", [(64, 3000, 0.026, 45.5, 64.0), (16, 3000, 0.0105, 11.6, 20.0),
+                                             (256, 4200, 0.1, 181.3, 256.0)])
+def test_source_beside_the_image_keeps_the_integral_form(vg, n, nu, du, DSO, DSD):
+    """Half widths within 1 % of DSO / sqrt(2): the call gives the integral form's bits."""
+    import torch
+    from vir_gb300 import _core, _lib
+    from vir_gb300.sys_mat import dd
+    angs = np.pi / 4 + np.linspace(0, 2 * np.pi, 8, endpoint=False)
+    x = torch.rand((n, n), generator=torch.Generator().manual_seed(3)).cuda()
+    xT, out = x.t().contiguous(), torch.empty((8, nu), device="cuda")
+    f = _core.f32
+    g = _lib.DD2DGeom(n, n, 8, nu, f(du), 0.0, 1.0, f(DSO), f(DSD), 1, 4)
+    _lib.call("vg_dd2d_fp", ctypes.byref(g), _core.ptr(x), _core.ptr(xT),
+              _core.ptr(_core.trig_cache.get(angs, np.float32, x.device)), _core.ptr(out), _core.stream(x.device))
+    assert torch.equal(dd.dd_fp_fan_2d(x, angs, nu, DSO, DSD, du=du), out)

@@ -657,7 +657,11 @@ __device__ __forceinline__ float tap_pairs(const float *__restrict__ px, const f
     const float z0 = (float)io + zofs;
     float2 z = make_float2(z0, z0 + 1.0f);
     const float2 A = dup(b.alpha), B = dup(b.beta), IW = dup(b.iw);
-    const float2 E = dup(FIRST ? -b.eps : b.eps), E1 = dup(FIRST ? 1.0f + b.eps : 1.0f - b.eps);
+    // FIRST: S = r (1 + eps - eps r) for r <= 1 and 1 beyond, where it falls again (a
+    // bin may be so narrow next to the source that eps r > 1 at the next pixel edge);
+    // -eps as the rest of the rounded 1 + eps, so that S is 1 exactly at r = 1
+    const float e1 = FIRST ? 1.0f + b.eps : 1.0f - b.eps;
+    const float2 E = dup(FIRST ? 1.0f - e1 : b.eps), E1 = dup(e1);
     int off = io * nd + kofs - TAP_BITS;  // pixel offset of the line less that of floor(x)'s bits
     const float4 *tp = tab + (io >> 1), *te = tab + (ie >> 1);
     while (tp < te) {
@@ -677,13 +681,17 @@ __device__ __forceinline__ float tap_pairs(const float *__restrict__ px, const f
             float2 r = pk_mul(g, q), v = V[N - 1];
 #pragma unroll
             for (int i = 1; i < N; ++i) {
-                float2 S = pk_fma(E, r, E1);
-                if (!FIRST) {
+                float2 S;
+                if (FIRST) {
+                    const float2 t1 = make_float2(fminf(r.x, 1.0f), fminf(r.y, 1.0f));
+                    S = pk_mul(t1, pk_fma(E, t1, E1));
+                } else {
+                    S = pk_fma(E, r, E1);
                     asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(S.x));
                     asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(S.y));
+                    S = pk_mul(r, S);
+                    S = make_float2(fminf(S.x, 1.0f), fminf(S.y, 1.0f));
                 }
-                S = pk_mul(r, S);
-                S = make_float2(fminf(S.x, 1.0f), fminf(S.y, 1.0f));
                 v = pk_fma(S, pk_fma(V[i], dup(-1.0f), V[i - 1]), v);
                 if (i + 1 < N) r = pk_add(r, q);
             }
@@ -1115,14 +1123,19 @@ int launch_fp_t(const vg_dd2d_geom *g, const float *img, const float *imgT, cons
 
 // Whether the tap form is the one for the geometry: fan beam, bins of about 1.5
 // pixels at most at the isocentre (wider ones, whose pixels it would read one by
-// one, are the integral form's), and the inverse map's pole so far off the
+// one, are the integral form's), the inverse map's pole so far off the
 // detector that positions stay exact to the fraction where a bin meets the image
-// (|x| < 2^21): den >= 0.07 DSD.
+// (|x| < 2^21): den >= 0.07 DSD, and no line nearer to the source of a diagonal view
+// than 0.18 of its distance: a bin is that much narrower on it, and the rounding of
+// its position that much more of it (16 to 200 pixels square, bins of 0.03 to 1
+// pixel, largest error against FP64 over that of the integral form: up to 1.1 at
+// 0.2, up to 4 at 0.15, 2.5 at 0.07).
 bool taps_serve(const vg_dd2d_geom *g) {
     if (!g->fan || (size_t)g->nx * g->ny >= (1u << 30)) return false;
     const double nm = g->nx > g->ny ? g->nx : g->ny, du = g->du, d = g->d_pix;
     const double ext = fmax(fabs(du * (-0.5 * g->nu + g->su)), fabs(du * (0.5 * g->nu + g->su)));
-    return du * g->DSO <= 1.5 * g->DSD * d && ext <= 0.9 * g->DSD && 12.8 * g->DSO / d + 14.0 * nm < 2e6;
+    return du * g->DSO <= 1.5 * g->DSD * d && ext <= 0.9 * g->DSD && 12.8 * g->DSO / d + 14.0 * nm < 2e6 &&
+           0.5 * (nm - 1.0) * d <= 0.82 * 0.70710678 * g->DSO;
 }
 
 // Forward projection variants: 1 .. FP_NVARIANTS - 1 the tiles of the integral
@@ -1160,7 +1173,8 @@ int launch_taps(const vg_dd2d_geom *g, const float *img, const float *imgT, cons
     while (LS > 1 && taps_smem(g, cb, LS) > TAP_SMEM) LS /= 2;
     const size_t smem = taps_smem(g, cb, LS);
     VG_REQUIRE(smem <= TAP_SMEM, "dd2d_fp: sizes too large for this variant");
-    // first order in eps leaves 0.15 eps^2 of a bin at a pixel edge: 1.3e-6 at most here
+    // first order in eps leaves 0.15 eps^2 of a bin at a pixel edge inside the bin
+    // (r < 1; the others need no share): 1.3e-6 at most here
     const float ext = fmaxf(fabsf(g->du * (0.f - 0.5f * g->nu + g->su)),
                             fabsf(g->du * ((float)g->nu - 0.5f * g->nu + g->su)));
     auto kern = g->du <= 3e-3f * (g->DSD - ext) ? dd2d_fp_taps_kernel<true> : dd2d_fp_taps_kernel<false>;
