@@ -64,7 +64,9 @@ class SIRT2D:
         _core.require_cuda()
         self.dev = device or _core.device_of(sino)
         self.fan = 1 if geom == "fan" else 0
-        self.y = _core.to_device(sino, self.dev)
+        y = _core.to_device(sino, self.dev)
+        # a buffer of its own: load_sino writes to it
+        self.y = y.clone() if _core.is_torch(sino) and y.data_ptr() == sino.data_ptr() else y
         self.trig = _core.trig_cache.get(ang_arr, np.float32, self.dev)
         na = self.trig.numel() // 2
         nx, ny = (int(v) for v in img_shape)
