@@ -40,6 +40,34 @@ def test_sf_cone_columns_vs_oracle(vg, orc, name):
         assert np.abs(got - ref).max() <= 5e-5 * np.abs(ref).max()
 
 
+# Last tiles of 1, 2, 5 and 6 columns (pairs without a live column), the same with
+# columns beside the detector, and magnifications of 1.4 to 3.5 in one tile, so that
+# columns over 5 and 6 u cells (per-voxel path) lie between narrower ones.
+PAIRS = {
+    "one": ((9, 7, 40), 40, 44, 21, 1.0, 1.0, 40.0, 70.0),
+    "two": ((10, 9, 70), 40, 64, 21, 1.0, 1.0, 40.0, 70.0),
+    "five": ((13, 8, 33), 45, 41, 21, 1.0, 1.0, 40.0, 70.0),
+    "six": ((14, 9, 66), 45, 72, 21, 1.0, 1.0, 40.0, 70.0),
+    "beside": ((21, 22, 34), 12, 40, 33, 1.0, 1.0, 40.0, 70.0),
+    "near": ((14, 13, 36), 60, 90, 33, 1.0, 1.2, 14.0, 28.0),
+}
+
+
+@pytest.mark.parametrize("name", sorted(PAIRS))
+def test_sf_bp_pairs_skipped_vs_oracle(vg, orc, name):
+    """Pairs of columns that use no row buffer, between and after ones that do."""
+    from vir_gb300.sys_mat import sp
+    shape, nu, nv, na, du, dv, DSO, DSD = PAIRS[name]
+    angs = np.linspace(0.05, 0.05 + 2 * np.pi, na, endpoint=False)
+    f = lambda v: float(np.float32(v))
+    kw = dict(du=f(du), dv=f(dv), su=0.25, sv=0.5, d_pix=1.0)
+    y = np.random.default_rng(29).random((na, nu, nv)).astype(np.float32)
+    ref = orc.sf_bp_cone_3d(y, angs, shape, DSO, DSD, **kw)
+    for _ in range(3):
+        got = sp.sf_bp_cone_3d(y, angs, shape, DSO, DSD, **kw)
+        assert np.abs(got - ref).max() <= 5e-5 * np.abs(ref).max()
+
+
 def test_sf_cone_columns_nan_stays_near(vg):
     """A NaN voxel or cell reaches only outputs within two of those it overlaps."""
     import torch

@@ -591,7 +591,12 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
             const char *q = reinterpret_cast<const char *>(qw + (size_t)(ib + sv) * g.nu * g.nv);
 #pragma unroll
             for (int c0 = 0; c0 < BT; c0 += 2) {
-                if (!(lv >> c0 & 3)) continue;
+                // every pair has a barrier, also one that uses no row buffer: it lies
+                // between the reads of the pair before and the next stores there
+                if (!(lv >> c0 & 3)) {
+                    __syncwarp();
+                    continue;
+                }
                 if (sl >> c0 & 3) {
                     const float2 cs = view_cs(trig, a0 + ib + sv);
 #pragma unroll
@@ -604,6 +609,7 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
                                                            vox(g.d_pix, x0 + c, g.nx),
                                                            vox(g.d_pix, iy, g.ny), iz);
                         }
+                    __syncwarp();
                     continue;
                 }
                 float (*T)[BW] = W.T[c0 >> 1 & 1];
