@@ -123,8 +123,8 @@ __device__ __forceinline__ void axis_start(Axis &a, const SidGeom &g, double o0,
     const long long ob = ord64(tb);
     // planes below the point at tb; the first one ahead of it
     const int below = __double2int_rd(fma(fma(tb, d, o0), g.inv_dpix, 0.5 * n));
-    int i = max(-1, min(n + 1, a.s > 0 ? min(below, n) + 1 : below));
-    if (a.s > 0 ? i < 0 : i > n) i -= a.s;  // the walk's first plane at the earliest
+    // (before the walk's first plane: that one; past its last: none is left)
+    int i = a.s > 0 ? max(min(below, n) + 1, 0) : min(max(below, -1), n);
     if ((unsigned)i <= (unsigned)n) {
         a.t = cross_at(a, g.d_pix, i, et);
         a.o = ord64(a.t);
