@@ -85,3 +85,23 @@ def test_sf_cone_columns_nan_stays_near(vg):
                 else torch.nn.functional.max_pool3d(near[None, None], 5, 1, 2)[0, 0]) > 0
         a.view(-1)[a.numel() // 2 + 7] = float("nan")
         assert not bool((torch.isnan(call(a)) & ~near).any())
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("nz,nv,du", [(32, 64, 1.0), (70, 63, 1.0), (40, 90, 0.45)])
+def test_sf_bp_nonfinite_cell_reaches_what_it_overlaps(vg, nz, nv, du, value):
+    """A cell that is not finite makes exactly the voxels non-finite that a
+    cell of 1 in its place reaches (1 and 2 groups of slices, 4- and 16-byte
+    loads, columns over up to and over more than 4 u cells)."""
+    import torch
+    from vir_gb300.sys_mat import sp
+    shape, nu, na = (13, 16, nz), 40, 6
+    angs = np.linspace(0.1, 0.1 + 2 * np.pi, na, endpoint=False)
+    bp = lambda t: sp.sf_bp_cone_3d(t, angs, shape, 60.0, 100.0, du=du, dv=1.03, su=0.31, sv=0.17, d_pix=1.0)
+    for at in ((1, 20, nv // 2), (4, 13, 2), (3, 0, nv - 1)):
+        y = torch.zeros((na, nu, nv), device="cuda")
+        y[at] = 1.0
+        near = bp(y) != 0
+        y = torch.rand((na, nu, nv), generator=torch.Generator().manual_seed(6)).cuda()
+        y[at] = value
+        assert torch.equal(~torch.isfinite(bp(y)), near)

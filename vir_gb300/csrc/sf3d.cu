@@ -504,6 +504,26 @@ __device__ __noinline__ float sf_voxel_view(const vg_dd3d_geom &g, const float *
     return part * inv_dv;
 }
 
+// views [ia, ie) of 8 columns (x0 + c, iy) and the slices z0 + lane + 32 i < z0 + sz,
+// voxel by voxel, added to their sums at kh
+__device__ __noinline__ void sf_views_again(const vg_dd3d_geom &g, const float *__restrict__ qw,
+                                            const double *__restrict__ trig, int a0, int ia, int ie, int x0, int iy,
+                                            int z0, int sz, float2 *kh) {
+    for (int c = 0; c < BT && x0 + c < g.nx && iy < g.ny; ++c)
+        for (int z = threadIdx.x & 31; z < sz && z0 + z < g.nz; z += 32) {
+            float t = 0.f;
+            for (int a = ia; a < ie; ++a) {
+                const float2 cs = view_cs(trig, a0 + a);
+                t += sf_voxel_view(g, qw + (size_t)a * g.nu * g.nv, cs.x, cs.y, vox(g.d_pix, x0 + c, g.nx),
+                                   vox(g.d_pix, iy, g.ny), z0 + z);
+            }
+            Kahan k;
+            k.s = kh[c * sz + z].x; k.c = kh[c * sz + z].y;
+            k.add(t);
+            kh[c * sz + z] = make_float2(k.s, k.c);
+        }
+}
+
 constexpr int SF_BP_MINB = 3;
 
 template <int VEC, int M>
@@ -531,18 +551,36 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
 #pragma unroll
         for (int m = 0; m < M; ++m) grp[c][m] = 0.f;
     int ngrp = 0;
-    auto flush = [&]() {
+    // the sums of the ngrp views before view ie
+    auto flush = [&](int ie) {
+        bool odd = false;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            float t = grp[0][m];
+#pragma unroll
+            for (int c = 1; c < BT; ++c) t += grp[c][m];
+            odd |= 32 * m + lane < zn && !(fabsf(t) < INFINITY);
+        }
+        // infinities and NaN only to the slices that their cells overlap: the v step
+        // multiplies cells of weight 0 too, so these views again, voxel by voxel
+        if (__any_sync(0xffffffffu, odd)) {
+            sf_views_again(g, qw, trig, a0, ie - ngrp, ie, x0, iy, z0, SZ, kh + BT * warp * SZ);
+        } else {
+#pragma unroll
+            for (int c = 0; c < BT; ++c)
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    float2 *k = kh + (c + BT * warp) * SZ + 32 * m + lane;
+                    Kahan a;
+                    a.s = k->x; a.c = k->y;
+                    a.add(grp[c][m]);
+                    *k = make_float2(a.s, a.c);
+                }
+        }
 #pragma unroll
         for (int c = 0; c < BT; ++c)
 #pragma unroll
-            for (int m = 0; m < M; ++m) {
-                float2 *k = kh + (c + BT * warp) * SZ + 32 * m + lane;
-                Kahan a;
-                a.s = k->x; a.c = k->y;
-                a.add(grp[c][m]);
-                *k = make_float2(a.s, a.c);
-                grp[c][m] = 0.f;
-            }
+            for (int m = 0; m < M; ++m) grp[c][m] = 0.f;
         ngrp = 0;
     };
     const int va0 = (int)((long long)cnt * rank / S), va1 = (int)((long long)cnt * (rank + 1) / S);
@@ -714,11 +752,10 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
                         grp[c0 + h][m] = a;
                     }
             }
-            if (++ngrp == BP_GROUP) flush();
+            if (++ngrp == BP_GROUP || ib + sv + 1 == va1) flush(ib + sv + 1);
         }
         __syncwarp();  // the table and the row buffers are reused
     }
-    flush();
     if (S > 1) cl.sync();
     else __syncthreads();
     for (int col = warp * S + rank; col < BT * BT; col += 8 * S) {
