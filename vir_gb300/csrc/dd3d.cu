@@ -173,8 +173,10 @@ __device__ __noinline__ float fp_cell_line(const vg_dd3d_geom &g, const View3 &v
 //      input column;
 //   v: every output adds its rows of that buffer, with v-overlaps that stay in
 //      registers for the line.
-// Rows are counted in input cells from the window's start, which is found in
-// FP64, so a cell edge is an integer.  The u-overlaps of 4 lines or views are
+// Rows are counted in input cells from the one at the middle of the tile's
+// outputs, which is found in FP64, so a cell edge is an integer and an output's
+// edge carries the rounding of its distance from there, however short the tile.
+// The u-overlaps of 4 lines or views are
 // tabulated at once (lane = line or view x column) in the warp's own shared
 // memory: the warps of a block do not wait for each other.
 //
@@ -188,7 +190,6 @@ __device__ __noinline__ float fp_cell_line(const vg_dd3d_geom &g, const View3 &v
 // side 11.0 ms; that layout on global loads 12.6 ms.
 constexpr int BT = 8;    // columns per warp
 constexpr int BW = 128;  // rows of one column buffer
-constexpr int MID = 40;  // rows are counted from here, about the middle: half the rounding of counts from 0
 constexpr int FP_GROUP = 16, BP_GROUP = 16;  // lines, views summed in registers before the running sum
 
 // a pair's columns start one input column apart and have 2-3 each
@@ -200,8 +201,36 @@ struct WarpBuf {
     float4 uw[4][BT];  // overlaps with 3 input columns, (bits) the first | count << 20
                        // | SHARED in a pair's first column
     float w3[4][BT];   // overlap with a fourth
-    float4 line[4];    // rows per output, first row - start - MID, start, falling input order
+    float4 line[4];    // of the v step, see Line
 };
+
+// The rows of zn outputs, b input rows each, the middle one (zn / 2) starting at row
+// t of the input (n rows): they are counted from row c = floor(t), and the window
+// that is staged starts at a multiple of 4 at or below the first output's row, found
+// with the expression of Strip::init.  Packed as (b, t - c, window's start + falling
+// input order, c - start | rows of the window << 12).
+struct Line {
+    float b, y;
+    int start, mid, rows;
+
+    // the outputs' rows fit a column buffer, and one output's NW
+    template <int NW>
+    __device__ __forceinline__ bool fits() const { return b <= NW - 1.0f && rows <= BW - NW + 1; }
+    __device__ __forceinline__ float4 pack(int rev) const {
+        return make_float4(b, y, __int_as_float(start + rev), __int_as_float(mid | rows << 12));
+    }
+};
+__device__ __forceinline__ Line line_at(double b, double t, int zn) {
+    Line l;
+    const int c = __double2int_rd(t);
+    const float lo = -(float)(zn >> 1);
+    l.b = (float)b;
+    l.y = (float)(t - c);
+    l.start = (c + __float2int_rd(fmaf(l.b, lo, l.y))) & ~3;
+    l.mid = c - l.start;
+    l.rows = l.mid + __float2int_rd(fmaf(l.b, (float)zn + lo, l.y)) + 1;
+    return l;
+}
 
 // One line and view of a warp.  VEC: floats per input load (4 needs input
 // columns that start on 16-byte boundaries).  M = 2 takes outputs of up to 2
@@ -217,34 +246,29 @@ struct Strip {
     int win;
     bool two;
 
-    // whether rows up to ve (excluded) fit a column buffer, and an output NW rows
-    static __device__ __forceinline__ bool fits(float4 ln, int ve) {
-        return ln.x <= NW - 1.0f && ve - __float_as_int(ln.z) <= BW - NW + 1;
-    }
-
-    // line record ln (see WarpBuf), rows up to ve of an input of n rows, zn outputs
-    __device__ __forceinline__ void init(const float *src, unsigned stride, int lane, float4 ln, int ve, int zn,
-                                         int n) {
-        const int vs = __float_as_int(ln.z), sw = __float_as_int(ln.w);
+    // packed Line ln, zn outputs, an input of n rows
+    __device__ __forceinline__ void init(const float *src, unsigned stride, int lane, float4 ln, int zn, int n) {
+        const int vs = __float_as_int(ln.z) & ~3, sw = __float_as_int(ln.z) & 1;
+        const int mid = __float_as_int(ln.w) & 0xfff;
         float over = 0.f;
         int qf[M];
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-            const float zm = (float)(32 * m + lane);
+            const float zm = (float)(32 * m + lane - (zn >> 1));
             const float tl = fmaf(ln.x, zm, ln.y), th = fmaf(ln.x, zm + 1.0f, ln.y);
             const float tf = floorf(tl);
             w[m][0] = fminf(th, tf + 1.0f) - tl;
 #pragma unroll
             for (int t = 1; t < NW; ++t) w[m][t] = __saturatef(th - (tf + (float)t));
             if (32 * m + lane < zn) over = fmaxf(over, th - tf);
-            qf[m] = (int)tf + MID;
+            qf[m] = (int)tf + mid;
             const int q = min(qf[m], BW - NW);  // outputs past the end read anything
             qa[m] = q + (sw ? BW : 0);
             qb[m] = q + (sw ? 0 : BW);
         }
         two = !__any_sync(0xffffffffu, over > 2.0f);
         // rows are clamped to the window and the input; rows outside it weigh nothing
-        win = ve - vs + NW - 1;
+        win = (__float_as_int(ln.w) >> 12) + NW - 1;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int v = vs + min(VEC == 4 ? 4 * lane : lane + 32 * i, (win - 1) & ~(VEC - 1));
@@ -424,7 +448,7 @@ dd3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const float4 *__re
     const size_t so = v.xdrv ? (size_t)g.nz : (size_t)g.ny * g.nz;  // stride of io
     const float inv_d = 1.0f / g.d_pix;
     const int zn = min(SZ, g.nv - v0);
-    const double vd = (double)v0 - 0.5 * g.nv + (double)g.sv;
+    const double vd = (double)(v0 + (zn >> 1)) - 0.5 * g.nv + (double)g.sv;  // the middle v cell's edge
     // this lane's u cell in the table (slot order: a pair's pixels ascending)
     const bool rev = v.pd < 0.f;
     const int ls = lane >> 3, cs = lane & 7, iu = u0 + (cs ^ (int)rev);
@@ -470,24 +494,24 @@ dd3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const float4 *__re
                     }
                 }
             }
-            wide4 = __ballot_sync(0xffffffffu, n > 4);
-            live4 = __ballot_sync(0xffffffffu, n > 0);
-            put_column(W, ls, cs, w, ks, n);
-            if (cs == 0 && io < no) {  // the tile's first slice: a multiple of 4 and the rest
-                const double b = __ldg(&bt[(size_t)ia * nm + io].y), t = fma(b, vd, 0.5 * g.nz);
-                const int zs = __double2int_rd(t) & ~3;
-                W.line[ls] = make_float4((float)b, (float)(t - (zs + MID)), __int_as_float(zs), __int_as_float(rev));
+            bool slow = n > 4, miss = false;
+            if (cs == 0 && io < no) {
+                const double b = __ldg(&bt[(size_t)ia * nm + io].y);
+                const Line l = line_at(b, fma(b, vd, 0.5 * g.nz), zn);
+                if (!l.fits<Strip<VEC, M>::NW>() || big) slow = true;
+                else miss = l.start + l.rows <= 0 || l.start >= g.nz;
+                W.line[ls] = l.pack(rev);
             }
+            wide4 = __ballot_sync(0xffffffffu, slow);
+            live4 = __ballot_sync(0xffffffffu, n > 0) & ~(__ballot_sync(0xffffffffu, miss) * 0xffu);
+            put_column(W, ls, cs, w, ks, n);
             __syncwarp();
         }
         const int nb = min(4, no - ib);
         for (int sv = 0; sv < nb; ++sv) {
             if (!(live4 >> (8 * sv) & 0xff)) continue;
-            const float4 ln = W.line[sv];
-            const int zs = __float_as_int(ln.z), ze = zs + __float2int_rd(fmaf(ln.x, (float)zn, ln.y)) + MID + 1;
-            if (ze <= 0 || zs >= g.nz) continue;
             const int io = ib + sv;
-            if ((wide4 >> (8 * sv) & 0xff) || !Strip<VEC, M>::fits(ln, ze) || big) {
+            if (wide4 >> (8 * sv) & 0xff) {
                 const float c = cen(g.d_pix, io, no);
                 const float cp = v.po * c, co = v.oo * c;
                 const float2 sz = __ldg(tab + (size_t)ia * nm + io);
@@ -503,7 +527,7 @@ dd3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const float4 *__re
                     }
             } else {
                 Strip<VEC, M> st;
-                st.init(vol + io * so, (unsigned)sk, lane, ln, ze, zn, g.nz);
+                st.init(vol + io * so, (unsigned)sk, lane, W.line[sv], zn, g.nz);
 #pragma unroll
                 for (int c0 = 0; c0 < BT; c0 += 2) st.pair(W, sv, c0, lane, grp[c0], grp[c0 + 1]);
             }
@@ -626,8 +650,8 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
     WarpBuf &W = reinterpret_cast<WarpBuf *>(kh + BT * BT * SZ)[warp];
     const int nm = g.nx > g.ny ? g.nx : g.ny;
     const float idu = 1.0f / g.du, u0 = ufloor_edge(g, 0);
-    const double zd = (double)z0 - 0.5 * g.nz, cv = 0.5 * g.nv - (double)g.sv;
     const int zn = min(SZ, g.nz - z0);
+    const double zd = (double)(z0 + (zn >> 1)) - 0.5 * g.nz, cv = 0.5 * g.nv - (double)g.sv;  // the middle slice's edge
     for (int i = tid; i < BT * BT * SZ; i += 256) kh[i] = make_float2(0.f, 0.f);
     __syncthreads();
     float grp[BT][M];
@@ -663,13 +687,15 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
             const int k = (v.xdrv ? x0 : y0) + c, io = (v.xdrv ? y0 : x0) + warp;
             float w[4] = {0.f, 0.f, 0.f, 0.f};
             int js = 0, nrow = 0;
+            bool slow = false, miss = false;
             if (io < no) {
                 const float2 sz = __ldg(tab + (size_t)ia * nm + io);
-                if (c == 0) {  // the tile's first row: a multiple of 4 and the rest
-                    const double b = __ldg(&bt[(size_t)ia * nm + io].x), t = fma(b, zd, cv);
-                    const int vs = __double2int_rd(t) & ~3;
-                    W.line[sv] = make_float4((float)b, (float)(t - (vs + MID)), __int_as_float(vs),
-                                             __int_as_float(v.pd < 0.f));
+                if (c == 0) {
+                    const double b = __ldg(&bt[(size_t)ia * nm + io].x);
+                    const Line l = line_at(b, fma(b, zd, cv), zn);
+                    if (!l.fits<Strip<VEC, M>::NW>()) slow = true;
+                    else miss = l.start + l.rows <= 0 || l.start >= g.nv;
+                    W.line[sv] = l.pack(v.pd < 0.f);
                 }
                 const float ce = cen(g.d_pix, io, no);
                 const float cp = v.po * ce, co = v.oo * ce;
@@ -686,8 +712,8 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
                 }
             }
             xdrv4 = __ballot_sync(0xffffffffu, v.xdrv);
-            wide4 = __ballot_sync(0xffffffffu, nrow > 4);
-            live4 = __ballot_sync(0xffffffffu, nrow > 0);
+            wide4 = __ballot_sync(0xffffffffu, slow || nrow > 4);
+            live4 = __ballot_sync(0xffffffffu, nrow > 0) & ~(__ballot_sync(0xffffffffu, miss) * 0xffu);
             put_column(W, sv, c ^ (int)(v.pd < 0.f), w, js, nrow);
             __syncwarp();
         }
@@ -703,11 +729,8 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
             }
             const bool live = (live4 >> (8 * sv)) & 0xff;
             if (live) {
-                const float4 ln = W.line[sv];
                 const float *s = sino + (size_t)ia * g.nu * g.nv;
-                const int vs = __float_as_int(ln.z);
-                const int ve = vs + __float2int_rd(fmaf(ln.x, (float)zn, ln.y)) + MID + 1;  // rows [vs, ve)
-                if ((wide4 >> (8 * sv) & 0xff) || !Strip<VEC, M>::fits(ln, ve)) {
+                if (wide4 >> (8 * sv) & 0xff) {
                     const View3 v = view_f(vf, ia);
                     const int nd = v.xdrv ? g.nx : g.ny, no = v.xdrv ? g.ny : g.nx;
                     const int io = (v.xdrv ? y0 : x0) + warp;
@@ -721,9 +744,9 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
                                 grp[c][m] += bp_voxel_view(g, v, s, __ldg(tab + (size_t)ia * nm + io),
                                                            k, nd, v.po * ce, v.oo * ce, iz);
                         }
-                } else if (ve > 0 && vs < g.nv) {
+                } else {
                     Strip<VEC, M> st;
-                    st.init(s, g.nv, lane, ln, ve, zn, g.nv);
+                    st.init(s, g.nv, lane, W.line[sv], zn, g.nv);
 #pragma unroll
                     for (int c0 = 0; c0 < BT; c0 += 2) st.pair(W, sv, c0, lane, grp[c0], grp[c0 + 1]);
                 }
