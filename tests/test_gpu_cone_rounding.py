@@ -40,3 +40,14 @@ def test_short_profiles_rounding(vg, orc, kind):
         e_bp.append(_unit(bp(y, ang, (1, 1, 4), DSO, DSD, **kw)) - _unit(obp(y, ang, (1, 1, 4), DSO, DSD, **kw)))
     for e in (e_fp, e_bp):
         assert np.linalg.norm(np.stack(e)) <= 4e-7 * np.sqrt(len(e))
+
+
+def test_output_just_below_a_slice_boundary(vg, orc):
+    """A tile of one output that starts 2^-25 of a slice below slice nz / 2, which
+    float32 rounds onto it."""
+    from vir_gb300.sys_mat import dd
+    vol = np.random.default_rng(3).random((1, 1, 160)).astype(np.float32)
+    kw = dict(du=16.0, dv=float(np.float32(5.0 / 3.0)), su=0.0, sv=0.5 - 2.0**-25, d_pix=1.0)
+    ref = orc.dd_fp_cone_3d(vol, np.array([0.0]), 1, 1, DSO, DSD, **kw)
+    got = dd.dd_fp_cone_3d(vol, np.array([0.0]), 1, 1, DSO, DSD, **kw)
+    assert np.abs(got - ref).max() <= 5e-5 * np.abs(ref).max()

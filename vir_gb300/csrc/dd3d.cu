@@ -225,7 +225,7 @@ __device__ __forceinline__ Line line_at(double b, double t, int zn) {
     const int c = __double2int_rd(t);
     const float lo = -(float)(zn >> 1);
     l.b = (float)b;
-    l.y = (float)(t - c);
+    l.y = fminf((float)(t - c), 0.99999994f);  // below 1, so that the start is at c at most
     l.start = (c + __float2int_rd(fmaf(l.b, lo, l.y))) & ~3;
     l.mid = c - l.start;
     l.rows = l.mid + __float2int_rd(fmaf(l.b, (float)zn + lo, l.y)) + 1;
