@@ -21,7 +21,7 @@ def _unit(a):
     return a / np.linalg.norm(a, axis=-1, keepdims=True)
 
 
-@pytest.mark.parametrize("kind", ["dd"])
+@pytest.mark.parametrize("kind", ["dd", "sf"])
 def test_short_profiles_rounding(vg, orc, kind):
     from vir_gb300.sys_mat import dd, sp
     fp, bp = (dd.dd_fp_cone_3d, dd.dd_bp_cone_3d) if kind == "dd" else (sp.sf_fp_cone_3d, sp.sf_bp_cone_3d)

@@ -145,7 +145,7 @@ __device__ __forceinline__ float unproj_idx(const vg_dd3d_geom &g, float c, floa
 // memory (one 16-byte load per 4 slices, the next column's issued before this
 // one is used), every lane sums its M v cells' 2-5 slices with their overlaps,
 // and adds the result to the cells the column covers.  Overlaps are counted in
-// slices from about the window's middle.  Lines with more than 32 columns, or
+// slices from the tile's middle.  Lines with more than 32 columns, or
 // v cells over more slices than a row buffer holds, take a per-cell path.  Sums:
 // 16 lines in registers, then a second running sum in shared memory.
 //
@@ -156,12 +156,35 @@ __device__ __forceinline__ float unproj_idx(const vg_dd3d_geom &g, float c, floa
 // per SM 21.6, 5 22.5, 6 22.4 ms.
 constexpr int SFW = 4, SF_FP_MINB = 4;  // warps per block
 constexpr int UC = 8;                   // u cells per warp
-constexpr int BW = 128, MID = 40;       // entries of a row buffer, and where their count starts
+constexpr int BW = 128;                 // entries of a row buffer
+
+// The entries of a column's zn outputs, B each, the middle one (zn / 2) at entry
+// ci + t of the input (t the product with B, ci + cf the offset): they are counted
+// from c = floor(t) + ci, so an output carries the rounding of its distance from the
+// middle; the window that is staged starts at or below the first output's entry,
+// found with the v step's expression.
+struct Win {
+    float y;               // the middle output from c on
+    int start, mid, rows;  // c - start, entries of the window
+};
+template <int VEC>
+__device__ __forceinline__ Win win_at(float B, float t, float cf, float ci, int zn) {
+    Win w;
+    const float tf = floorf(t), lo = -(float)(zn >> 1), u = fminf(t - tf, 0.99999994f) + cf, uf = floorf(u);
+    const int c = (int)tf + (int)ci + (int)uf;
+    w.y = u - uf;  // below 1, so that the start is at c at most
+    w.start = c + __float2int_rd(fmaf(B, lo, w.y));
+    if (VEC == 4) w.start &= ~3;
+    w.mid = c - w.start;
+    w.rows = w.mid + __float2int_rd(fmaf(B, (float)zn + lo, w.y)) + 1;
+    return w;
+}
 
 struct SfFpWarp {
     float T[2][BW];
     float w[32][UC];  // per column: F1 l_phi0 M d / dv on the u cells
-    float4 rec[32];   // slices per v cell, first slice - start - MID, start, index of the column
+    float4 rec[32];   // slices per v cell, Win's y and start, index of the column
+    int mr[32];       // Win's mid | rows << 12
 };
 
 // one cell's share of one line, straight from global memory (any geometry)
@@ -213,7 +236,7 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
         pole = up >= TUa - 2.f * g.du && up <= TUb + 2.f * g.du;
     }
     const float kB = g.dv / (g.DSD * g.d_pix);  // slices per v cell = kB (DSO - o)
-    const float vd = (float)v0 - 0.5f * g.nv + g.sv;
+    const float vd = (float)(v0 + (zn >> 1)) - 0.5f * g.nv + g.sv;  // the middle v cell's edge
     const float ci = floorf(0.5f * g.nz), cf = 0.5f * g.nz - ci;
     float2 grp[UC / 2][M];  // u cells in pairs
 #pragma unroll
@@ -253,8 +276,9 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
             if (!slow) {
                 // this lane's column
                 float w[UC];
-                float B = 1.f, first = 0.f;
-                int zs = 0, cidx = 0;
+                float B = 1.f;
+                Win r = {};
+                int cidx = 0;
                 bool any = false, bad = false;
                 if (ka + lane <= ke) {
                     const int k = ka + lane;
@@ -272,13 +296,9 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
                             e = t;
                         }
                         B = kB * (g.DSO - fmaf(c, x, s * y));
-                        const float t = B * vd, tf = floorf(t);
-                        const int fl = (int)tf + (int)ci;
-                        zs = VEC == 4 ? fl & ~3 : fl;
-                        first = (t - tf) + cf + (float)(fl - zs - MID);
-                        const int ze = zs + __float2int_rd(fmaf(B, (float)zn, first)) + MID + 1;
-                        if (ze <= 0 || zs >= g.nz) any = false;
-                        bad = any && (B > NW - 1.0f || ze - zs > BW - NW + 1);
+                        r = win_at<VEC>(B, B * vd, cf, ci, zn);
+                        if (r.start + r.rows <= 0 || r.start >= g.nz) any = false;
+                        bad = any && (B > NW - 1.0f || r.rows > BW - NW + 1);
                         cidx = xdrv ? k * g.ny + io : io * g.ny + k;
                     }
                 }
@@ -287,7 +307,8 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
                 if (any) {
                     *reinterpret_cast<float4 *>(&W.w[lane][0]) = make_float4(w[0], w[1], w[2], w[3]);
                     *reinterpret_cast<float4 *>(&W.w[lane][4]) = make_float4(w[4], w[5], w[6], w[7]);
-                    W.rec[lane] = make_float4(B, first, __int_as_float(zs), __int_as_float(cidx));
+                    W.rec[lane] = make_float4(B, r.y, __int_as_float(r.start), __int_as_float(cidx));
+                    W.mr[lane] = r.mid | r.rows << 12;
                 }
                 __syncwarp();
             }
@@ -308,11 +329,13 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
                 int win = 0;
                 float2 r[2];
                 float4 rc;
+                int mr;
                 unsigned in = 0;
                 auto load = [&](int t) {  // column t's slices that this lane loads, clamped to the volume
                     rc = W.rec[t];
+                    mr = W.mr[t];
                     const int zs = __float_as_int(rc.z);
-                    win = __float2int_rd(fmaf(rc.x, (float)zn, rc.y)) + MID + NW;
+                    win = (mr >> 12) + NW - 1;
                     const char *p = ptr_at(reinterpret_cast<const char *>(vol), __float_as_int(rc.w), 4u * g.nz);
                     in = 0;
                     auto at = [&](int i) {
@@ -353,6 +376,7 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
                     }
                     __syncwarp();
                     const float4 cur = rc;
+                    const int mid = mr & 0xfff;
                     const float4 wa = *reinterpret_cast<const float4 *>(&W.w[t][0]);
                     const float4 wb = *reinterpret_cast<const float4 *>(&W.w[t][4]);
                     cols &= cols - 1;
@@ -365,10 +389,10 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
                     bool odd = false;
 #pragma unroll
                     for (int m = 0; m < M; ++m) {
-                        const float vm = (float)(32 * m + lane);
+                        const float vm = (float)(32 * m + lane - (zn >> 1));
                         const float tl = fmaf(cur.x, vm, cur.y), th = fmaf(cur.x, vm + 1.0f, cur.y);
                         const float tf = floorf(tl);
-                        const float *q = T + min((int)tf + MID, BW - NW);  // v cells past the detector read anything
+                        const float *q = T + min((int)tf + mid, BW - NW);  // v cells past the detector read anything
                         float a = (fminf(th, tf + 1.0f) - tl) * q[0];
                         a = fmaf(__saturatef(th - (tf + 1.0f)), q[1], a);
 #pragma unroll
@@ -461,7 +485,7 @@ __global__ void sf3d_weight(vg_dd3d_geom g, const float *__restrict__ sino, int 
 //      v cells its slices project to (16-byte loads, lane = 4 cells), into a row
 //      buffer in shared memory;
 //   v: lets every slice add its 2-5 cells of the buffer with their overlaps.
-// Overlaps are in cell units, counted from about the window's middle.  Sums: 16
+// Overlaps are in cell units, counted from the tile's middle.  Sums: 16
 // views in registers, then a compensated sum per voxel in shared memory.
 // Columns over more than 4 u cells, or whose slices reach more cells than the
 // buffer holds, take a per-voxel path.  With too few tiles to fill the GPU the
@@ -476,7 +500,7 @@ constexpr int BP_GROUP = 16;
 struct SfBpWarp {
     float T[2][2][BW];
     float4 w[4][BT];    // F1 l_phi0 / dv of u cells j0 .. j0 + 3
-    float4 rec[4][BT];  // v cells per slice, first cell - start - MID, start, j0 | count << 21
+    float4 rec[4][BT];  // v cells per slice, Win's y and start, j0 | count << 21 | Win's mid << 24
 };
 
 // one voxel, one view, straight from the weighted sinogram (any geometry)
@@ -540,7 +564,8 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
     SfBpWarp &W = reinterpret_cast<SfBpWarp *>(kh + BT * BT * SZ)[warp];
     const int iy = y0 + warp, zn = min(SZ, g.nz - z0);
     const float inv_du = 1.0f / g.du, U0 = uedge(g, 0);
-    const float zd = (float)z0 - 0.5f * g.nz;  // exact
+    const float zd = (float)(z0 + (zn >> 1)) - 0.5f * g.nz;  // the middle slice's edge, exact
+    const float hi = (float)(zn - (zn >> 1));
     const float cv = 0.5f * g.nv - g.sv, ci = floorf(cv), cf = cv - ci;  // cell coordinate of v = 0
     for (int c = warp; c < BT * BT; c += 8)
         for (int m = 0; m < M; ++m) kh[c * SZ + 32 * m + lane] = make_float2(0.f, 0.f);
@@ -590,8 +615,9 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
             const int sv = lane >> 3, c = lane & 7, ix = x0 + c;
             const float2 cs = view_cs(trig, a0 + min(ib + sv, cnt - 1));
             float w[BKU] = {0.f, 0.f, 0.f, 0.f};
-            float B = 1.f, first = 0.f;
-            int j0 = 0, n = 0, vs = 0;
+            float B = 1.f;
+            Win r = {};
+            int j0 = 0, n = 0;
             bool far = false;
             if (ix < g.nx && iy < g.ny) {
                 const SfCol C = sf_col(g, cs.x, cs.y, vox(g.d_pix, ix, g.nx), vox(g.d_pix, iy, g.ny));
@@ -608,19 +634,15 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
                     e = h;
                 }
                 B = C.mz / g.dv;
-                const float t = B * zd, tf = floorf(t);
-                const int fl = (int)tf + (int)ci;
-                vs = VEC == 4 ? fl & ~3 : fl;
-                first = (t - tf) + cf + (float)(fl - vs - MID);
-                const int ve = vs + __float2int_rd(fmaf(B, (float)zn, first)) + MID + 1;
-                far = ve <= 0 || vs >= g.nv;
-                if (B > NW - 1.0f || ve - vs > BW - NW + 1) n = n > 0 ? BKU + 1 : 0;
+                r = win_at<VEC>(B, B * zd, cf, ci, zn);
+                far = r.start + r.rows <= 0 || r.start >= g.nv;
+                if (B > NW - 1.0f || r.rows > BW - NW + 1) n = n > 0 ? BKU + 1 : 0;
             }
             if (far) n = 0;
             slow = __ballot_sync(0xffffffffu, n > BKU);
             live = __ballot_sync(0xffffffffu, n > 0);
             W.w[sv][c] = make_float4(w[0], w[1], w[2], w[3]);
-            W.rec[sv][c] = make_float4(B, first, __int_as_float(vs), __int_as_float(j0 | n << 21));
+            W.rec[sv][c] = make_float4(B, r.y, __int_as_float(r.start), __int_as_float(j0 | n << 21 | r.mid << 24));
             __syncwarp();
         }
         const int nb = min(4, va1 - ib);
@@ -658,9 +680,10 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const float4 w = W.w[sv][c0 + h], rc = W.rec[sv][c0 + h];
-                    const int vs = __float_as_int(rc.z), bits = __float_as_int(rc.w), n = bits >> 21;
+                    const int vs = __float_as_int(rc.z);
+                    const unsigned bits = __float_as_uint(rc.w), n = bits >> 21 & 7, mid = bits >> 24;
                     const unsigned j = bits & 0x1fffff;  // nu < 2^21
-                    const int win = __float2int_rd(fmaf(rc.x, (float)zn, rc.y)) + MID + NW;
+                    const int win = __float2int_rd(fmaf(rc.x, hi, rc.y)) + mid + NW;
                     // this lane's cells, clamped to the window and the detector
                     int vo[NV];
                     unsigned in = 0;
@@ -712,14 +735,14 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
                     float over = 0.f;
 #pragma unroll
                     for (int m = 0; m < M; ++m) {
-                        const float zm = (float)(32 * m + lane);
+                        const float zm = (float)(32 * m + lane - (zn >> 1));
                         const float tl = fmaf(rc.x, zm, rc.y), th = fmaf(rc.x, zm + 1.0f, rc.y);
                         const float tf = floorf(tl);
                         wv[h][m][0] = fminf(th, tf + 1.0f) - tl;
 #pragma unroll
                         for (int t = 1; t < NW; ++t) wv[h][m][t] = __saturatef(th - (tf + (float)t));
                         if (32 * m + lane < zn) over = fmaxf(over, th - tf);
-                        qi[h][m] = min((int)tf + MID, BW - NW);  // slices past the volume read anything
+                        qi[h][m] = min((int)tf + (int)mid, BW - NW);  // slices past the volume read anything
                     }
                     two[h] = !__any_sync(0xffffffffu, over > 2.0f);
                     if (VEC == 4) {
