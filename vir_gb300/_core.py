@@ -68,7 +68,7 @@ def ptr(t: torch.Tensor) -> int:
 
 
 def stream(dev=None) -> ctypes.c_void_p:
-    if dev is None or dev.index is None:
+    if not isinstance(dev, torch.device) or dev.index is None:  # None, "cuda:0", 0, "cuda"
         return ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
     # the same handle without building a Stream object (5 us)
     return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(dev.index))
