@@ -81,8 +81,14 @@ def _write(d):
 def _key(g, dev):
     name = torch.cuda.get_device_name(dev).replace(" ", "_")
     na_class = 1 << max(0, int(np.ceil(np.log2(max(g.na, 1)))))
+    # geometries that the tap form serves (the last variant, which the others are timed
+    # against) are a class of their own: an entry from before it was there, or of a
+    # geometry of these sizes that it does not serve, says nothing about them
+    L = load()
+    plain = DD2DGeom(g.nx, g.ny, g.na, g.nu, g.du, g.su, g.d_pix, g.DSO, g.DSD, g.fan, 0)
+    taps = L.vg_dd2d_fp_default_variant(ctypes.byref(plain)) == L.vg_dd2d_fp_variants()
     return (f"dd2d_fp|fan={g.fan}|nx={g.nx}|ny={g.ny}|nu={g.nu}|na~{na_class}|{name}"
-            f"|lib={load().vg_version()}")
+            f"|lib={L.vg_version()}" + ("|taps" if taps else ""))
 
 
 def time_fp_variants(g, dev, reps=3):
