@@ -1178,8 +1178,8 @@ int launch_taps(const vg_dd2d_geom *g, const float *img, const float *imgT, cons
     const float ext = fmaxf(fabsf(g->du * (0.f - 0.5f * g->nu + g->su)),
                             fabsf(g->du * ((float)g->nu - 0.5f * g->nu + g->su)));
     auto kern = g->du <= 3e-3f * (g->DSD - ext) ? dd2d_fp_taps_kernel<true> : dd2d_fp_taps_kernel<false>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) {  // to one limit for all sizes: other threads launch this kernel with theirs
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAP_SMEM);
         if (e != cudaSuccess) return cuda_status(e, "dd2d_fp: shared memory attribute");
     }
     dim3 grid(ceil_div(g->nu, cb), g->na);

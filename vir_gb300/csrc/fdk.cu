@@ -240,10 +240,11 @@ template <int H>
 int fdk_bp_launch(const vg_dd3d_geom *g, const float *q, const double *trig, float *vol, void *stream) {
     const float scale = (float)(3.14159265358979323846 / (2.0 * g->na));
     const size_t smem = (size_t)g->na * sizeof(float2);
-    VG_REQUIRE(smem <= 200 * 1024, "fdk_bp: more than 25600 views");
-    if (smem > 40 * 1024) {
+    constexpr size_t limit = 200 * 1024;
+    VG_REQUIRE(smem <= limit, "fdk_bp: more than 25600 views");
+    if (smem > 40 * 1024) {  // to one limit for all sizes: other threads launch this kernel with theirs
         cudaError_t e = cudaFuncSetAttribute(fdk_bp_kernel<H>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
         if (e != cudaSuccess) return cuda_status(e, "fdk_bp: shared memory attribute");
     }
     dim3 grid(ceil_div(g->nz, 64 * H), ceil_div(g->ny, FDK_COLS), g->nx);

@@ -176,9 +176,11 @@ extern "C" int vg_filter_rows_fft(const float *in, int rows, int nu, int z, cons
                "filter_rows_fft: z must be a power of two in [max(2 nu, 4), 32768]");
     const int N = z / 2;
     const size_t smem = (size_t)(2 * (N + (N >> 4)) + N) * sizeof(float2);
-    if (smem > 48 * 1024) {
+    if (smem > 48 * 1024) {  // to one limit for all sizes that fit (z = 16384 the largest): other
+                             // threads launch this kernel with theirs
+        const size_t limit = smem > 200 * 1024 ? smem : 200 * 1024;
         cudaError_t e = cudaFuncSetAttribute(filter_fft_kernel,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
         if (e != cudaSuccess) return cuda_status(e, "filter_rows_fft: shared memory attribute");
     }
     int L = 0;
