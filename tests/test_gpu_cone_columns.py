@@ -80,3 +80,35 @@ def test_cone_columns_unaligned_and_nonfinite(vg):
             near = torch.nn.functional.max_pool2d(near.float()[:, None], 5, 1, 2)[:, 0] > 0
         a.view(-1)[a.numel() // 2 + 7] = float("nan")
         assert not bool((torch.isnan(call(a)) & ~near).any())
+
+
+# shape, nu, nv, na, du, dv, d_pix, DSO, DSD: u cells over many pixels and voxels over
+# many detector columns (4 at a time), rows longer than a buffer (in pieces of 128), both,
+# a detector that reaches the pole of the inverse edge map, one cell for everything
+WIDE = {
+    "u": ((40, 38, 33), 9, 40, 7, 12.0, 1.4, 1.0, 60.0, 100.0),
+    "u_fine": ((9, 12, 64), 500, 70, 7, 0.1, 1.3, 1.0, 40.0, 70.0),
+    "v": ((9, 8, 301), 21, 7, 7, 1.2, 33.0, 0.5, 60.0, 110.0),
+    "v_fine": ((7, 9, 40), 24, 900, 5, 1.2, 0.09, 0.9, 40.0, 70.0),
+    "uv": ((30, 28, 150), 5, 5, 9, 16.0, 41.0, 1.0, 60.0, 100.0),
+    "uv_fine": ((6, 7, 9), 300, 400, 5, 0.11, 0.12, 1.0, 30.0, 55.0),
+    "pole": ((20, 24, 10), 60, 30, 16, 5.0, 1.5, 1.0, 60.0, 100.0),
+    "all": ((12, 10, 90), 1, 1, 8, 400.0, 4000.0, 1.0, 60.0, 100.0),
+}
+
+
+@pytest.mark.parametrize("name", sorted(WIDE))
+def test_cone_columns_wide_vs_oracle(vg, orc, name):
+    from vir_gb300.sys_mat import dd
+    shape, nu, nv, na, du, dv, d, DSO, DSD = WIDE[name]
+    rng = np.random.default_rng(19)
+    angs = _angles(na, "shuffled")
+    f = lambda v: float(np.float32(v))
+    kw = dict(du=f(du), dv=f(dv), su=f(0.3), sv=f(-0.4), d_pix=f(d))
+    vol = rng.random(shape).astype(np.float32)
+    y = rng.random((na, nu, nv)).astype(np.float32)
+    for got, ref in ((dd.dd_fp_cone_3d(vol, angs, nu, nv, DSO, DSD, **kw),
+                      orc.dd_fp_cone_3d(vol, angs, nu, nv, DSO, DSD, **kw)),
+                     (dd.dd_bp_cone_3d(y, angs, shape, DSO, DSD, **kw),
+                      orc.dd_bp_cone_3d(y, angs, shape, DSO, DSD, **kw))):
+        assert np.abs(got - ref).max() <= 5e-5 * np.abs(ref).max()

@@ -208,16 +208,17 @@ struct WarpBuf {
 // t of the input (n rows): they are counted from row c = floor(t), and the window
 // that is staged starts at a multiple of 4 at or below the first output's row, found
 // with the expression of Strip::init.  Packed as (b, t - c, window's start + falling
-// input order, c - start | rows of the window << 12).
+// input order, c - start | rows of the window << 12), or, where the rows do not fit a
+// column buffer or one output's NW, (b, t - c, falling input order, c) for long_pair.
 struct Line {
     float b, y;
     int start, mid, rows;
 
-    // the outputs' rows fit a column buffer, and one output's NW
     template <int NW>
     __device__ __forceinline__ bool fits() const { return b <= NW - 1.0f && rows <= BW - NW + 1; }
-    __device__ __forceinline__ float4 pack(int rev) const {
-        return make_float4(b, y, __int_as_float(start + rev), __int_as_float(mid | rows << 12));
+    __device__ __forceinline__ float4 pack(int rev, bool fit) const {
+        return make_float4(b, y, __int_as_float(fit ? start + rev : rev),
+                           __int_as_float(fit ? mid | rows << 12 : start + mid));
     }
 };
 __device__ __forceinline__ Line line_at(double b, double t, int zn) {
@@ -257,7 +258,7 @@ struct Strip {
             const float zm = (float)(32 * m + lane - (zn >> 1));
             const float tl = fmaf(ln.x, zm, ln.y), th = fmaf(ln.x, zm + 1.0f, ln.y);
             const float tf = floorf(tl);
-            w[m][0] = fminf(th, tf + 1.0f) - tl;
+            w[m][0] = fminf(ln.x, (tf + 1.0f) - tl);  // all of an output inside one row: its size, unrounded
 #pragma unroll
             for (int t = 1; t < NW; ++t) w[m][t] = __saturatef(th - (tf + (float)t));
             if (32 * m + lane < zn) over = fmaxf(over, th - tf);
@@ -409,26 +410,83 @@ struct Strip {
 };
 
 // Table entry of one output column (lane, slot = its place in input order
-// within a pair): n input columns from js on with overlaps w.
-__device__ __forceinline__ void put_column(WarpBuf &W, int sv, int slot, const float (&w)[4], int js, int n) {
+// within a pair): n <= 4 input columns from js on with overlaps w.
+__device__ __forceinline__ void put_column(WarpBuf &W, int sv, int slot, const float (&w)[4], int js, int n,
+                                           bool store = true) {
     const int js2 = __shfl_xor_sync(0xffffffffu, js, 1), n2 = __shfl_xor_sync(0xffffffffu, n, 1);
     const bool shared = !(slot & 1) && js2 == js + 1 && (n & ~1) == 2 && (n2 & ~1) == 2;
-    W.uw[sv][slot] = make_float4(w[0], w[1], w[2], __int_as_float(js | min(n, 5) << 20 | (shared ? SHARED : 0)));
+    if (!store) return;
+    W.uw[sv][slot] = make_float4(w[0], w[1], w[2], __int_as_float(js | n << 20 | (shared ? SHARED : 0)));
     W.w3[sv][slot] = w[3];
+}
+
+// A pair's outputs on a line whose rows do not fit Strip: the rows in pieces of a
+// column buffer, every output over its rows of each piece.
+template <int M>
+struct LongPair {
+    float a[M], b[M];  // of output columns c and c + 1
+};
+template <int M>
+__device__ __noinline__ LongPair<M> long_pair(WarpBuf &W, int sv, int c, const float *src, size_t stride, int zn,
+                                              int n) {
+    const int lane = threadIdx.x & 31;
+    const float4 ln = W.line[sv];
+    const int rev = __float_as_int(ln.z) & 1, mid = max(min(__float_as_int(ln.w), 1 << 29), -(1 << 29));
+    const auto at = [&](int z) {  // output z's first edge, from row mid on
+        return fminf(fmaxf(fmaf(ln.x, (float)(z - (zn >> 1)), ln.y), -1073741824.f), 1073741824.f);
+    };
+    const auto row = [&](int z) { return mid + __float2int_rd(at(z)); };
+    LongPair<M> p;
+#pragma unroll
+    for (int m = 0; m < M; ++m) p.a[m] = p.b[m] = 0.f;
+    const int r1 = min(row(zn) + 1, n);
+    for (int r0 = max(row(0), 0); r0 < r1; r0 += BW) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float4 e = W.uw[sv][c + h];
+            const int bits = __float_as_int(e.w), nc = bits >> 20 & 7;
+            const float *q = src + (size_t)(bits & 0xfffff) * stride;
+            const float w[4] = {e.x, e.y, e.z, W.w3[sv][c + h]};
+            for (int i = lane; i < BW; i += 32) {
+                float o = 0.f;
+                if (r0 + i < r1)
+                    for (int t = 0; t < nc; ++t) o = fmaf(w[t], __ldg(q + t * stride + (r0 + i)), o);
+                W.T[0][h][i] = o;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const int z = 32 * m + lane;
+            if (z >= zn) continue;
+            const float tl = at(z), th = at(z + 1);
+            const int e = min(min(mid + __float2int_rd(th) + 1, r0 + BW), r1);
+            for (int r = max(row(z), r0); r < e; ++r) {
+                const float x = (float)(r - mid), ov = fminf(th, x + 1.0f) - fmaxf(tl, x);
+                if (ov > 0.f) {
+                    p.a[m] = fmaf(ov, W.T[0][rev][r - r0], p.a[m]);
+                    p.b[m] = fmaf(ov, W.T[0][rev ^ 1][r - r0], p.b[m]);
+                }
+            }
+        }
+        __syncwarp();
+    }
+    return p;
 }
 
 // Forward projection.  Block = one view, 32 u cells x 32 M v cells; a warp
 // owns 8 u cells and walks the lines of the volume, 4 at a time.  The pixel
 // columns under a u cell come from the exact inverse of the edge projection.
-// Lines where a u cell overlaps more than 4 pixels, or the tile's v cells more
-// slices than a column buffer holds, take the per-cell global path.  Sums: 16
+// WIDE: lines where a u cell overlaps more than 4 pixels take 4 at a time, those
+// where the tile's v cells overlap more slices than a column buffer holds long_pair;
+// else such lines, few then, take the per-cell global path.  Sums: 16
 // lines in registers, then a second running sum in shared memory.  At 128
 // registers 4 blocks of 4 warps fit an SM: 13.1 ms at 256^3 (5 blocks, with
 // spills, 13.8 ms; 3 15.0 ms); with 64 v cells per warp 16.0 ms.
 constexpr int FPW = 4;       // warps per block
 constexpr int FP_MINB = 4;
 // MODE 0: projection; 1: SIRT residual epilogue
-template <int MODE, int VEC, int M>
+template <int MODE, int VEC, int M, bool WIDE>
 __global__ void __launch_bounds__(32 * FPW, FP_MINB)
 dd3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const float4 *__restrict__ vf,
                const float2 *__restrict__ tab, const double2 *__restrict__ bt, float *__restrict__ sino,
@@ -464,54 +522,61 @@ dd3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const float4 *__re
             grp[c][m] = 0.f;
             acc[c * SZ + 32 * m] = 0.f;
         }
+    // pixels under this lane's u cell on line io: their number, and from the k0-th on the
+    // overlaps with 4 and the first of those
+    auto columns = [&](int io, int k0, float (&w)[4], int &ks) {
+        int n = 0;
+        ks = 0;
+        w[0] = w[1] = w[2] = w[3] = 0.f;
+        if (io < no && cell) {
+            const float c = cen(g.d_pix, io, no);
+            const float cp = v.po * c, co = v.oo * c;
+            const float2 sz = __ldg(tab + (size_t)ia * nm + io);
+            const float a = fmaf(Ul, g.DSO - co, -g.DSD * cp) * rl * inv_d + 0.5f * nd;
+            const float b = fmaf(Ur, g.DSO - co, -g.DSD * cp) * rr * inv_d + 0.5f * nd;
+            const float fl = fminf(a, b), fh = fmaxf(a, b);
+            ks = pole ? 0 : (int)floorf(fminf(fmaxf(fl, 0.f), (float)(nd - 1)));
+            n = pole ? nd : fh >= 0.f && fl < (float)nd ? min((int)floorf(fh), nd - 1) - ks + 1 : 0;
+            if (k0 > 0) ks = n > k0 ? ks + k0 : 0;
+            float pa = projU(g, v, cp, co, edg(g.d_pix, ks, nd));
+            const float sc = sz.x * sz.y * g.d_pix;  // v-overlaps are in slices
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const float pb = projU(g, v, cp, co, edg(g.d_pix, ks + t + 1, nd));
+                const float o = fminf(fmaxf(pa, pb), Ur) - fmaxf(fminf(pa, pb), Ul);
+                w[t] = (k0 + t < n && o > 0.f) ? o * sc : 0.f;
+                pa = pb;
+            }
+        }
+        return n;
+    };
     int ngrp = 0;
     for (int ib = 0; ib < no; ib += 4) {
-        unsigned wide4, live4;
+        unsigned wide4, long4, live4;
         {
             const int io = ib + ls;
-            float w[4] = {0.f, 0.f, 0.f, 0.f};
-            int ks = 0, n = 0;
-            if (io < no && cell) {
-                const float c = cen(g.d_pix, io, no);
-                const float cp = v.po * c, co = v.oo * c;
-                const float2 sz = __ldg(tab + (size_t)ia * nm + io);
-                const float a = fmaf(Ul, g.DSO - co, -g.DSD * cp) * rl * inv_d + 0.5f * nd;
-                const float b = fmaf(Ur, g.DSO - co, -g.DSD * cp) * rr * inv_d + 0.5f * nd;
-                const float fl = fminf(a, b), fh = fmaxf(a, b);
-                if (pole) {
-                    n = 5;
-                } else {
-                    ks = (int)floorf(fminf(fmaxf(fl, 0.f), (float)(nd - 1)));
-                    n = fh >= 0.f && fl < (float)nd ? min((int)floorf(fh), nd - 1) - ks + 1 : 0;
-                    float pa = projU(g, v, cp, co, edg(g.d_pix, ks, nd));
-                    const float sc = sz.x * sz.y * g.d_pix;  // v-overlaps are in slices
-#pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        const float pb = projU(g, v, cp, co, edg(g.d_pix, ks + t + 1, nd));
-                        const float o = fminf(fmaxf(pa, pb), Ur) - fmaxf(fminf(pa, pb), Ul);
-                        w[t] = (t < n && o > 0.f) ? o * sc : 0.f;
-                        pa = pb;
-                    }
-                }
-            }
-            bool slow = n > 4, miss = false;
+            float w[4];
+            int ks;
+            const int n = columns(io, 0, w, ks);
+            bool fit = true, miss = false;
             if (cs == 0 && io < no) {
                 const double b = __ldg(&bt[(size_t)ia * nm + io].y);
                 const Line l = line_at(b, fma(b, vd, 0.5 * g.nz), zn);
-                if (!l.fits<Strip<VEC, M>::NW>() || big) slow = true;
-                else miss = l.start + l.rows <= 0 || l.start >= g.nz;
-                W.line[ls] = l.pack(rev);
+                fit = l.fits<Strip<VEC, M>::NW>() && !big;
+                miss = fit && (l.start + l.rows <= 0 || l.start >= g.nz);
+                W.line[ls] = l.pack(rev, fit);
             }
-            wide4 = __ballot_sync(0xffffffffu, slow);
+            wide4 = __ballot_sync(0xffffffffu, n > 4 || (!WIDE && !fit));
+            long4 = WIDE ? __ballot_sync(0xffffffffu, !fit) : 0;
             live4 = __ballot_sync(0xffffffffu, n > 0) & ~(__ballot_sync(0xffffffffu, miss) * 0xffu);
-            put_column(W, ls, cs, w, ks, n);
+            put_column(W, ls, cs, w, ks, min(n, 4));
             __syncwarp();
         }
         const int nb = min(4, no - ib);
         for (int sv = 0; sv < nb; ++sv) {
             if (!(live4 >> (8 * sv) & 0xff)) continue;
             const int io = ib + sv;
-            if (wide4 >> (8 * sv) & 0xff) {
+            if (!WIDE && (wide4 >> (8 * sv) & 0xff)) {
                 const float c = cen(g.d_pix, io, no);
                 const float cp = v.po * c, co = v.oo * c;
                 const float2 sz = __ldg(tab + (size_t)ia * nm + io);
@@ -526,10 +591,38 @@ dd3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const float4 *__re
                                                              vfloor_edge(g, iv), vfloor_edge(g, iv + 1));
                     }
             } else {
-                Strip<VEC, M> st;
-                st.init(vol + io * so, (unsigned)sk, lane, W.line[sv], zn, g.nz);
+                // the next 4 pixels of the cells over more than k0
+                auto more = [&](int k0) {
+                    if (!WIDE || !(wide4 >> (8 * sv) & 0xff)) return false;
+                    float w[4];
+                    int ks;
+                    const int n = columns(io, k0, w, ks);
+                    __syncwarp();
+                    put_column(W, sv, cs, w, ks, max(min(n - k0, 4), 0), ls == sv);
+                    __syncwarp();
+                    return __any_sync(0xffffffffu, n > k0) != 0;
+                };
+                int k0 = 0;
+                if (WIDE && (long4 >> (8 * sv) & 1)) {
+                    do {
 #pragma unroll
-                for (int c0 = 0; c0 < BT; c0 += 2) st.pair(W, sv, c0, lane, grp[c0], grp[c0 + 1]);
+                        for (int c0 = 0; c0 < BT; c0 += 2) {
+                            const LongPair<M> p = long_pair<M>(W, sv, c0, vol + io * so, sk, zn, g.nz);
+#pragma unroll
+                            for (int m = 0; m < M; ++m) {
+                                grp[c0][m] += p.a[m];
+                                grp[c0 + 1][m] += p.b[m];
+                            }
+                        }
+                    } while (more(k0 += 4));
+                } else {
+                    do {
+                        Strip<VEC, M> st;
+                        st.init(vol + io * so, (unsigned)sk, lane, W.line[sv], zn, g.nz);
+#pragma unroll
+                        for (int c0 = 0; c0 < BT; c0 += 2) st.pair(W, sv, c0, lane, grp[c0], grp[c0 + 1]);
+                    } while (more(k0 += 4));
+                }
             }
             if (++ngrp == FP_GROUP) {
 #pragma unroll
@@ -562,17 +655,31 @@ dd3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const float4 *__re
         }
 }
 
-template <int MODE, int VEC, int M>
+template <int MODE, int VEC, int M, bool WIDE>
 int launch_fp_t(const vg_dd3d_geom *g, const float *vol, const Ws3 &w, float *sino, const float *y,
                 const float *inv_w, cudaStream_t st) {
     constexpr size_t smem = FPW * (BT * 32 * M * sizeof(float) + sizeof(WarpBuf));
-    int s = cuda_status(cudaFuncSetAttribute(dd3d_fp_kernel<MODE, VEC, M>,
+    int s = cuda_status(cudaFuncSetAttribute(dd3d_fp_kernel<MODE, VEC, M, WIDE>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                         "dd3d_fp");
     if (s) return s;
     dim3 grid(ceil_div(g->nv, 32 * M), ceil_div(g->nu, BT * FPW), g->na);
-    dd3d_fp_kernel<MODE, VEC, M><<<grid, 32 * FPW, smem, st>>>(*g, vol, w.vf, w.tab, w.bt, sino, y, inv_w);
+    dd3d_fp_kernel<MODE, VEC, M, WIDE><<<grid, 32 * FPW, smem, st>>>(*g, vol, w.vf, w.tab, w.bt, sino, y, inv_w);
     return launch_status("dd3d_fp");
+}
+
+template <int MODE, bool WIDE>
+int launch_fp_w(const vg_dd3d_geom *g, const float *vol, const Ws3 &w, float *sino, const float *y,
+                const float *inv_w, int M, cudaStream_t st) {
+    const bool vec = g->nz % 4 == 0 && ((uintptr_t)vol & 15) == 0;
+    switch (M) {
+        case 3: return vec ? launch_fp_t<MODE, 4, 3, WIDE>(g, vol, w, sino, y, inv_w, st)
+                           : launch_fp_t<MODE, 1, 3, WIDE>(g, vol, w, sino, y, inv_w, st);
+        case 2: return vec ? launch_fp_t<MODE, 4, 2, WIDE>(g, vol, w, sino, y, inv_w, st)
+                           : launch_fp_t<MODE, 1, 2, WIDE>(g, vol, w, sino, y, inv_w, st);
+        default: return vec ? launch_fp_t<MODE, 4, 1, WIDE>(g, vol, w, sino, y, inv_w, st)
+                            : launch_fp_t<MODE, 1, 1, WIDE>(g, vol, w, sino, y, inv_w, st);
+    }
 }
 
 template <int MODE>
@@ -583,15 +690,20 @@ int launch_fp(const vg_dd3d_geom *g, const float *vol, const Ws3 &w, float *sino
     // detector's last tile is emptier for it
     const double r = 0.5 * hypot((double)g->nx, (double)g->ny) * g->d_pix;
     const double bmax = (g->DSO + r) / g->DSD * g->dv / g->d_pix;
-    const bool vec = g->nz % 4 == 0 && ((uintptr_t)vol & 15) == 0;
+    int M = 1;
     if (g->nv > 32 && 96.0 * bmax + 9.0 <= BW && 96 * ceil_div(g->nv, 96) <= 1.15 * 64 * ceil_div(g->nv, 64))
-        return vec ? launch_fp_t<MODE, 4, 3>(g, vol, w, sino, y, inv_w, st)
-                   : launch_fp_t<MODE, 1, 3>(g, vol, w, sino, y, inv_w, st);
-    if (g->nv > 32 && 64.0 * bmax + 9.0 <= BW)
-        return vec ? launch_fp_t<MODE, 4, 2>(g, vol, w, sino, y, inv_w, st)
-                   : launch_fp_t<MODE, 1, 2>(g, vol, w, sino, y, inv_w, st);
-    return vec ? launch_fp_t<MODE, 4, 1>(g, vol, w, sino, y, inv_w, st)
-               : launch_fp_t<MODE, 1, 1>(g, vol, w, sino, y, inv_w, st);
+        M = 3;
+    else if (g->nv > 32 && 64.0 * bmax + 9.0 <= BW)
+        M = 2;
+    // 32 where that leaves few blocks (200 of 64 v cells, 200^3 and 4 views: 0.33 ms, of
+    // 32 cells 0.30; 288, 128^3 and 16 views: 0.221 against 0.228)
+    if ((long long)ceil_div(g->nv, 32 * M) * ceil_div(g->nu, BT * FPW) * g->na < 250) M = 1;
+    // WIDE from u cells of 3.2 pixels on, by the widest at the far side of the volume
+    // (128^3, 120 views: 0.65 against 0.78 ms at 3.0, 1.44 against 0.77 at 3.4), and
+    // where rows do not fit (v cells of 4 slices, 180 views: 3.8 against 2.4 ms)
+    const bool wide = 32.0 * M * bmax + 9.0 > BW || 1.415 * (g->DSO + r) / g->DSD * g->du / g->d_pix > 3.2;
+    return wide ? launch_fp_w<MODE, true>(g, vol, w, sino, y, inv_w, M, st)
+                : launch_fp_w<MODE, false>(g, vol, w, sino, y, inv_w, M, st);
 }
 
 // Backprojection.  Block = 8 x 8 columns (x, y) x 32 M slices; a warp owns one
@@ -599,8 +711,9 @@ int launch_fp(const vg_dd3d_geom *g, const float *vol, const Ws3 &w, float *sino
 // the views, 4 at a time.  Its warps wait for each other only where the
 // driving axis changes and a voxel's sum moves to another warp.  Sums: 16
 // views in registers, then a compensated sum per voxel in shared memory.
-// Lines whose voxels cover more than 4 detector columns, or more rows than a
-// column buffer holds, take the per-voxel global path.  With too few tiles to
+// Lines whose voxels cover more than 4 detector columns, or more rows than a column
+// buffer holds, take the per-voxel global path; WIDE, where such columns are many and
+// the rows fit, takes 4 columns at a time.  With too few tiles to
 // fill the GPU, a cluster of up to 8 blocks shares a tile, each with a part of
 // the views; their sums are added in rank order through distributed shared
 // memory.  At 80 registers 3 blocks fit an SM (256^3: 9.3 ms; 2 blocks of 128
@@ -635,7 +748,7 @@ __device__ float bp_voxel_view(const vg_dd3d_geom &g, const View3 &v, const floa
 
 // MODE 0: back projection; 1: SIRT update epilogue.  VEC: floats per sinogram
 // load (4 needs nv % 4 == 0 and a 16-byte aligned sinogram).
-template <int MODE, int VEC, int M>
+template <int MODE, int VEC, int M, bool WIDE>
 __global__ void __launch_bounds__(256, VG_CONE_BP_MINB)
 dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__restrict__ vf,
                const float2 *__restrict__ tab, const double2 *__restrict__ bt, float *__restrict__ vol,
@@ -675,46 +788,57 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
         }
         ngrp = 0;
     };
+    const int ls = lane >> 3, cs = lane & 7;
+    // detector columns under voxel column cs of the warp's line in view ia: their number,
+    // and from the k0-th on the overlaps with 4 and the first of those
+    auto columns = [&](int ia, const View3 &v, int k0, float (&w)[4], int &js) {
+        const int nd = v.xdrv ? g.nx : g.ny, no = v.xdrv ? g.ny : g.nx;
+        const int k = (v.xdrv ? x0 : y0) + cs, io = (v.xdrv ? y0 : x0) + warp;
+        int n = 0;
+        js = 0;
+        w[0] = w[1] = w[2] = w[3] = 0.f;
+        if (io < no) {
+            const float sc = __ldg(tab + (size_t)ia * nm + io).x * g.dv;
+            const float ce = cen(g.d_pix, io, no);
+            const float cp = v.po * ce, co = v.oo * ce;
+            const float pa = projU(g, v, cp, co, edg(g.d_pix, k, nd));
+            const float pb = projU(g, v, cp, co, edg(g.d_pix, k + 1, nd));
+            const float ulo = fminf(pa, pb), uhi = fmaxf(pa, pb);
+            js = max((int)floorf((ulo - u0) * idu), 0);
+            n = k < nd ? max(min((int)floorf((uhi - u0) * idu), g.nu - 1) - js + 1, 0) : 0;
+            js = min(js, g.nu - 1);
+            if (k0 > 0) js = n > k0 ? js + k0 : 0;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const float o = fminf(uhi, ufloor_edge(g, js + t + 1)) - fmaxf(ulo, ufloor_edge(g, js + t));
+                w[t] = (k0 + t < n && o > 0.f) ? o * sc : 0.f;
+            }
+        }
+        return n;
+    };
     const int va0 = (int)((long long)g.na * rank / S), va1 = (int)((long long)g.na * (rank + 1) / S);
     for (int ib = va0; ib < va1; ib += 4) {
         // u-overlaps of views ib .. ib + 3 (lane = view * 8 + column)
         unsigned xdrv4, wide4, live4;
         {
-            const int sv = lane >> 3, c = lane & 7;
-            const int ia = min(ib + sv, g.na - 1);
+            const int ia = min(ib + ls, g.na - 1);
             const View3 v = view_f(vf, ia);
-            const int nd = v.xdrv ? g.nx : g.ny, no = v.xdrv ? g.ny : g.nx;
-            const int k = (v.xdrv ? x0 : y0) + c, io = (v.xdrv ? y0 : x0) + warp;
-            float w[4] = {0.f, 0.f, 0.f, 0.f};
-            int js = 0, nrow = 0;
-            bool slow = false, miss = false;
-            if (io < no) {
-                const float2 sz = __ldg(tab + (size_t)ia * nm + io);
-                if (c == 0) {
-                    const double b = __ldg(&bt[(size_t)ia * nm + io].x);
-                    const Line l = line_at(b, fma(b, zd, cv), zn);
-                    if (!l.fits<Strip<VEC, M>::NW>()) slow = true;
-                    else miss = l.start + l.rows <= 0 || l.start >= g.nv;
-                    W.line[sv] = l.pack(v.pd < 0.f);
-                }
-                const float ce = cen(g.d_pix, io, no);
-                const float cp = v.po * ce, co = v.oo * ce;
-                const float pa = projU(g, v, cp, co, edg(g.d_pix, k, nd));
-                const float pb = projU(g, v, cp, co, edg(g.d_pix, k + 1, nd));
-                const float ulo = fminf(pa, pb), uhi = fmaxf(pa, pb);
-                js = max((int)floorf((ulo - u0) * idu), 0);
-                nrow = k < nd ? max(min((int)floorf((uhi - u0) * idu), g.nu - 1) - js + 1, 0) : 0;
-                js = min(js, g.nu - 1);
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const float o = fminf(uhi, ufloor_edge(g, js + t + 1)) - fmaxf(ulo, ufloor_edge(g, js + t));
-                    w[t] = (t < nrow && o > 0.f) ? o * (sz.x * g.dv) : 0.f;
-                }
+            float w[4];
+            int js;
+            const int n = columns(ia, v, 0, w, js);
+            bool fit = true, miss = false;
+            const int io = (v.xdrv ? y0 : x0) + warp;
+            if (cs == 0 && io < (v.xdrv ? g.ny : g.nx)) {
+                const double b = __ldg(&bt[(size_t)ia * nm + io].x);
+                const Line l = line_at(b, fma(b, zd, cv), zn);
+                fit = l.fits<Strip<VEC, M>::NW>();
+                miss = fit && (l.start + l.rows <= 0 || l.start >= g.nv);
+                W.line[ls] = l.pack(v.pd < 0.f, true);
             }
             xdrv4 = __ballot_sync(0xffffffffu, v.xdrv);
-            wide4 = __ballot_sync(0xffffffffu, slow || nrow > 4);
-            live4 = __ballot_sync(0xffffffffu, nrow > 0) & ~(__ballot_sync(0xffffffffu, miss) * 0xffu);
-            put_column(W, sv, c ^ (int)(v.pd < 0.f), w, js, nrow);
+            wide4 = __ballot_sync(0xffffffffu, n > 4 || (!WIDE && !fit));
+            live4 = __ballot_sync(0xffffffffu, n > 0) & ~(__ballot_sync(0xffffffffu, miss) * 0xffu);
+            put_column(W, ls, cs ^ (int)(v.pd < 0.f), w, js, min(n, 4));
             __syncwarp();
         }
         const int nb = min(4, va1 - ib);
@@ -730,7 +854,7 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
             const bool live = (live4 >> (8 * sv)) & 0xff;
             if (live) {
                 const float *s = sino + (size_t)ia * g.nu * g.nv;
-                if (wide4 >> (8 * sv) & 0xff) {
+                if (!WIDE && (wide4 >> (8 * sv) & 0xff)) {
                     const View3 v = view_f(vf, ia);
                     const int nd = v.xdrv ? g.nx : g.ny, no = v.xdrv ? g.ny : g.nx;
                     const int io = (v.xdrv ? y0 : x0) + warp;
@@ -745,10 +869,25 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
                                                            k, nd, v.po * ce, v.oo * ce, iz);
                         }
                 } else {
-                    Strip<VEC, M> st;
-                    st.init(s, g.nv, lane, W.line[sv], zn, g.nv);
+                    // the next 4 detector columns of the voxels over more than k0
+                    auto more = [&](int k0) {
+                        if (!WIDE || !(wide4 >> (8 * sv) & 0xff)) return false;
+                        const View3 v = view_f(vf, ia);
+                        float w[4];
+                        int js;
+                        const int n = columns(ia, v, k0, w, js);
+                        __syncwarp();
+                        put_column(W, sv, cs ^ (int)(v.pd < 0.f), w, js, max(min(n - k0, 4), 0), ls == sv);
+                        __syncwarp();
+                        return __any_sync(0xffffffffu, n > k0) != 0;
+                    };
+                    int k0 = 0;
+                    do {
+                        Strip<VEC, M> st;
+                        st.init(s, g.nv, lane, W.line[sv], zn, g.nv);
 #pragma unroll
-                    for (int c0 = 0; c0 < BT; c0 += 2) st.pair(W, sv, c0, lane, grp[c0], grp[c0 + 1]);
+                        for (int c0 = 0; c0 < BT; c0 += 2) st.pair(W, sv, c0, lane, grp[c0], grp[c0 + 1]);
+                    } while (more(k0 += 4));
                 }
             }
             if (++ngrp == BP_GROUP) flush();
@@ -791,15 +930,21 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
     if (S > 1) cl.sync();  // no block leaves while its sums are read
 }
 
-constexpr size_t bp_smem(int M) { return (size_t)BT * BT * 32 * M * sizeof(float2) + 8 * sizeof(WarpBuf); }
-
-template <int MODE, int VEC, int M>
-int launch_bp_t(const vg_dd3d_geom *g, const float *sino, const Ws3 &w, float *vol, const float *inv_w, float gamma, cudaStream_t st) {
-    const long long tiles = (long long)ceil_div(g->nz, 32 * M) * ceil_div(g->ny, BT) * ceil_div(g->nx, BT);
-    // a cluster per tile until every SM has about three blocks, 16 views per block at least
+// Blocks of a cluster that share a tile: until every SM has about three blocks, 16
+// views per block at least.
+int bp_split(const vg_dd3d_geom *g, long long tiles) {
     int S = 1;
     while (S < 8 && tiles * S < 3 * 152 && g->na >= 32 * S) S *= 2;
-    int s = cuda_status(cudaFuncSetAttribute(dd3d_bp_kernel<MODE, VEC, M>,
+    return S;
+}
+
+constexpr size_t bp_smem(int M) { return (size_t)BT * BT * 32 * M * sizeof(float2) + 8 * sizeof(WarpBuf); }
+
+template <int MODE, int VEC, int M, bool WIDE>
+int launch_bp_t(const vg_dd3d_geom *g, const float *sino, const Ws3 &w, float *vol, const float *inv_w, float gamma, cudaStream_t st) {
+    const long long tiles = (long long)ceil_div(g->nz, 32 * M) * ceil_div(g->ny, BT) * ceil_div(g->nx, BT);
+    const int S = bp_split(g, tiles);
+    int s = cuda_status(cudaFuncSetAttribute(dd3d_bp_kernel<MODE, VEC, M, WIDE>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)bp_smem(M)), "dd3d_bp");
     if (s) return s;
@@ -813,23 +958,39 @@ int launch_bp_t(const vg_dd3d_geom *g, const float *sino, const Ws3 &w, float *v
     at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     c.attrs = at;
     c.numAttrs = 1;
-    return cuda_status(cudaLaunchKernelEx(&c, dd3d_bp_kernel<MODE, VEC, M>, *g, sino, w.vf, w.tab, w.bt, vol,
+    return cuda_status(cudaLaunchKernelEx(&c, dd3d_bp_kernel<MODE, VEC, M, WIDE>, *g, sino, w.vf, w.tab, w.bt, vol,
                                           inv_w, gamma), "dd3d_bp");
+}
+
+template <int MODE, bool WIDE>
+int launch_bp_w(const vg_dd3d_geom *g, const float *sino, const Ws3 &w, float *vol, const float *inv_w,
+                float gamma, bool two, cudaStream_t st) {
+    const bool vec = g->nv % 4 == 0 && ((uintptr_t)sino & 15) == 0;
+    if (two) return vec ? launch_bp_t<MODE, 4, 2, WIDE>(g, sino, w, vol, inv_w, gamma, st)
+                        : launch_bp_t<MODE, 1, 2, WIDE>(g, sino, w, vol, inv_w, gamma, st);
+    return vec ? launch_bp_t<MODE, 4, 1, WIDE>(g, sino, w, vol, inv_w, gamma, st)
+               : launch_bp_t<MODE, 1, 1, WIDE>(g, sino, w, vol, inv_w, gamma, st);
 }
 
 template <int MODE>
 int launch_bp(const vg_dd3d_geom *g, const float *sino, const Ws3 &w, float *vol, const float *inv_w,
               float gamma, cudaStream_t st) {
-    // 64 slices per warp while the rows they project to fit a column buffer,
-    // by the largest magnification a line of the volume can have
+    // 64 slices per warp while the rows they project to fit a column buffer, by the
+    // largest magnification a line of the volume can have -- also where the last tile is
+    // then emptier (96 x 96 x 65, 300 views: 0.70 ms, with 32 0.77) -- and there are
+    // about as many blocks as SMs (64^3, 8 views: 64 blocks 28.7 us, 128 of 32 slices 24.6)
     const double r = 0.5 * hypot((double)g->nx, (double)g->ny) * g->d_pix;
-    const double bmax = g->DSD / (g->DSO - fmin(r, 0.999 * g->DSO)) * g->d_pix / g->dv;
-    const bool two = g->nz > 32 && 64.0 * bmax + 9.0 <= BW;
-    const bool vec = g->nv % 4 == 0 && ((uintptr_t)sino & 15) == 0;
-    if (two) return vec ? launch_bp_t<MODE, 4, 2>(g, sino, w, vol, inv_w, gamma, st)
-                        : launch_bp_t<MODE, 1, 2>(g, sino, w, vol, inv_w, gamma, st);
-    return vec ? launch_bp_t<MODE, 4, 1>(g, sino, w, vol, inv_w, gamma, st)
-               : launch_bp_t<MODE, 1, 1>(g, sino, w, vol, inv_w, gamma, st);
+    const double mag = g->DSD / (g->DSO - fmin(r, 0.999 * g->DSO)), bmax = mag * g->d_pix / g->dv;
+    const long long tiles = (long long)ceil_div(g->nz, 64) * ceil_div(g->ny, BT) * ceil_div(g->nx, BT);
+    const bool two = g->nz > 32 && 64.0 * bmax + 9.0 <= BW && tiles * bp_split(g, tiles) >= 100;
+    // WIDE from voxels of 4.6 detector columns on, by the widest at the near side (128^3,
+    // 120 views: 0.57 against 0.62 ms at 4.4, 1.12 against 0.73 at 5.4).  Where rows do
+    // not fit the per-voxel path is the faster (slices over 4 v cells, 180 views: 3.8
+    // against 4.9 ms by long_pair, with voxels over 4 columns too 4.6 against 5.8)
+    const bool fit = two || 32.0 * bmax + 9.0 <= BW;  // then so on every line
+    const bool wide = fit && 1.415 * mag * g->d_pix / g->du > 4.6;
+    return wide ? launch_bp_w<MODE, true>(g, sino, w, vol, inv_w, gamma, two, st)
+                : launch_bp_w<MODE, false>(g, sino, w, vol, inv_w, gamma, two, st);
 }
 
 int check(const vg_dd3d_geom *g) {
