@@ -380,7 +380,8 @@ int vg_dd3d_bp(const vg_dd3d_geom *g, const float *sino, const double *trig,
  * through the column centre, l_theta = sqrt(1 + v^2 / (u^2 + DSD^2)) at the
  * cell centre.
  * vg_sf3d_fp: sino (na, nu, nv) = the line integrals above, gather form;
- *   workspace: nx ny (nz + 1) floats, checked but not used.
+ *   workspace: nx ny (nz + 1) floats, running sums of the volume over z where v
+ *   cells cover more than about 3.7 slices (asked for in every geometry).
  * vg_sf3d_bp: vol = its exact adjoint; workspace: the l_theta-weighted
  *   sinogram of a chunk of views (at most 256 MiB or one view).
  * Both take vg_sf3d_workspace_bytes(g) bytes (the larger need), 4-byte

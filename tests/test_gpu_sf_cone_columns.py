@@ -105,3 +105,47 @@ def test_sf_bp_nonfinite_cell_reaches_what_it_overlaps(vg, nz, nv, du, value):
         y = torch.rand((na, nu, nv), generator=torch.Generator().manual_seed(6)).cuda()
         y[at] = value
         assert torch.equal(~torch.isfinite(bp(y)), near)
+
+
+# shape, nu, nv, na, du, dv, d_pix, DSO, DSD: lines of more than 32 and 64 columns under 8
+# u cells, v cells over 4 to 40 slices (pieces of 240 rows), both, one cell for everything,
+# a detector that reaches the pole of the inverse edge map
+FP_WIDE = {
+    "u": ((90, 80, 20), 9, 30, 5, 18.0, 1.5, 1.0, 100.0, 160.0),
+    "v4": ((9, 8, 160), 21, 33, 7, 1.2, 4.4, 0.5, 60.0, 110.0),
+    "v40": ((8, 10, 500), 20, 9, 5, 1.2, 40.0, 0.5, 60.0, 110.0),
+    "uv": ((40, 36, 250), 7, 5, 6, 17.0, 60.0, 1.0, 60.0, 100.0),
+    "all": ((12, 10, 90), 1, 1, 8, 400.0, 4000.0, 1.0, 60.0, 100.0),
+    "pole": ((40, 36, 10), 60, 30, 16, 5.0, 1.5, 1.0, 60.0, 100.0),
+}
+
+
+@pytest.mark.parametrize("name", sorted(FP_WIDE))
+def test_sf_fp_wide_vs_oracle(vg, orc, name):
+    from vir_gb300.sys_mat import sp
+    shape, nu, nv, na, du, dv, d, DSO, DSD = FP_WIDE[name]
+    angs = np.linspace(0.03, 0.03 + 2 * np.pi, na, endpoint=False)
+    f = lambda v: float(np.float32(v))
+    kw = dict(du=f(du), dv=f(dv), su=f(0.3), sv=f(-0.4), d_pix=f(d))
+    vol = np.random.default_rng(31).random(shape).astype(np.float32)
+    got = sp.sf_fp_cone_3d(vol, angs, nu, nv, DSO, DSD, **kw)
+    ref = orc.sf_fp_cone_3d(vol, angs, nu, nv, DSO, DSD, **kw)
+    assert np.abs(got - ref).max() <= 5e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_sf_fp_long_cells_nonfinite_voxel(vg, value):
+    """Where v cells take running sums, a voxel that is not finite makes exactly the cells
+    non-finite that a voxel of 1 in its place reaches."""
+    import torch
+    from vir_gb300.sys_mat import sp
+    shape, nu, nv, na = (14, 16, 160), 24, 13, 6
+    angs = np.linspace(0.1, 0.1 + 2 * np.pi, na, endpoint=False)
+    fp = lambda t: sp.sf_fp_cone_3d(t, angs, nu, nv, 60.0, 100.0, du=1.1, dv=13.3, su=0.31, sv=0.17, d_pix=0.7)
+    for at in ((3, 9, 80), (13, 0, 1), (7, 7, 158)):
+        x = torch.zeros(shape, device="cuda")
+        x[at] = 1.0
+        near = fp(x) != 0
+        x = torch.rand(shape, generator=torch.Generator().manual_seed(6)).cuda()
+        x[at] = value
+        assert torch.equal(~torch.isfinite(fp(x)), near)

@@ -59,7 +59,7 @@ __device__ __forceinline__ float vox(float d, int i, int n) { return d * ((float
 // Footprint of column (x, y): sorted corner projections, l_phi0 and the
 // slice height on the detector M d.
 struct SfCol {
-    float t0, t1, t2, t3, lphi, mz, inv_mz;
+    float t0, t1, t2, t3, lphi, mz;
 };
 
 __device__ __forceinline__ void cswap(float &a, float &b) {
@@ -87,7 +87,6 @@ __device__ __forceinline__ SfCol sf_col(const vg_dd3d_geom &g, float c, float s,
     const float rx = x - g.DSO * c, ry = y - g.DSO * s;
     C.lphi = __fdividef(g.d_pix * sqrtf(rx * rx + ry * ry), fmaxf(fabsf(rx), fabsf(ry)));
     C.mz = __fdividef(g.DSD * g.d_pix, g.DSO - fmaf(c, x, s * y));
-    C.inv_mz = __fdividef(g.DSO - fmaf(c, x, s * y), g.DSD * g.d_pix);
     return C;
 }
 
@@ -105,22 +104,6 @@ __device__ __forceinline__ float trap_cum(float u, const SfCol &C) {
 // F1 averaged over [ua, ub] (cell width du), times l_phi0
 __device__ __forceinline__ float uweight(const SfCol &C, float ua, float ub, float inv_du) {
     return (trap_cum(ub, C) - trap_cum(ua, C)) * inv_du * C.lphi;
-}
-
-// sum_z f(z) |[M d (z - nz/2), M d (z + 1 - nz/2)] ∩ [va, vb]| / dv for one
-// column (f at col, slices contiguous)
-__device__ __forceinline__ float vprofile(const vg_dd3d_geom &g, const float *__restrict__ col,
-                                          float mz, float inv_mz, float va, float vb, float inv_dv) {
-    const float hz = 0.5f * g.nz;
-    const float sa = fmaf(va, inv_mz, hz), sb = fmaf(vb, inv_mz, hz);
-    const int z0 = max((int)floorf(sa), 0), z1 = min((int)floorf(sb), g.nz - 1);
-    float acc = 0.f;
-    for (int z = z0; z <= z1; ++z) {
-        const float lo = fmaxf(va, mz * ((float)z - hz)), hi = fminf(vb, mz * ((float)z + 1.f - hz));
-        const float ov = hi - lo;
-        if (ov > 0.f) acc = fmaf(__ldg(col + z), ov, acc);
-    }
-    return acc * inv_dv;
 }
 
 // Fractional pixel index, along the driving axis, of the point of the line
@@ -145,8 +128,10 @@ __device__ __forceinline__ float unproj_idx(const vg_dd3d_geom &g, float c, floa
 // memory (one 16-byte load per 4 slices, the next column's issued before this
 // one is used), every lane sums its M v cells' 2-5 slices with their overlaps,
 // and adds the result to the cells the column covers.  Overlaps are counted in
-// slices from the tile's middle.  Lines with more than 32 columns, or
-// v cells over more slices than a row buffer holds, take a per-cell path.  Sums:
+// slices from the tile's middle.  LONG: v cells over more slices than a row buffer
+// holds; every lane takes its cells' sums from running sums of the column (128^3, 180
+// views, v cells of 4, 6 and 10 slices: 1.5, 0.97 and 0.97 ms; cell by cell from the
+// volume 9.1, 9.6 and 11.4; the slices through the row buffer 3.1, 1.9 and 2.0).  Sums:
 // 16 lines in registers, then a second running sum in shared memory.
 //
 // Bound by instruction issue (72 %, 213 per column and line for 8 x 96 cells).
@@ -154,7 +139,7 @@ __device__ __forceinline__ float unproj_idx(const vg_dd3d_geom &g, float c, floa
 // in block-wide tables, one barrier per line (144 instructions per 32 cells and
 // line); the weights by branches per lane and the FMAs by cell 28 ms.  4 blocks
 // per SM 21.6, 5 22.5, 6 22.4 ms.
-constexpr int SFW = 4, SF_FP_MINB = 4;  // warps per block
+constexpr int SFW = 4, SF_FP_MINB = 4, SF_LONG_MINB = 6;  // warps per block
 constexpr int UC = 8;                   // u cells per warp
 constexpr int BW = 128;                 // entries of a row buffer
 
@@ -187,31 +172,56 @@ struct SfFpWarp {
     int mr[32];       // Win's mid | rows << 12
 };
 
-// one cell's share of one line, straight from global memory (any geometry)
-__device__ __noinline__ float sf_cell_line(const vg_dd3d_geom &g, const float *__restrict__ vol,
-                                           float c, float s, bool xdrv, int nd, int no, int io,
-                                           int kA, int kB, float Ua, float Ub, float Va, float Vb) {
-    const float inv_du = 1.0f / g.du, inv_dv = 1.0f / g.dv;
-    const float cen = vox(g.d_pix, io, no);
-    float part = 0.f;
-    for (int k = kA; k <= kB; ++k) {
-        const float b = vox(g.d_pix, k, nd);
-        const float x = xdrv ? b : cen, y = xdrv ? cen : b;
-        const SfCol C = sf_col(g, c, s, x, y);
-        if (C.t3 <= Ua || C.t0 >= Ub) continue;
-        const float w = uweight(C, Ua, Ub, inv_du);
-        if (w == 0.f) continue;
-        const int ix = xdrv ? k : io, iy = xdrv ? io : k;
-        part = fmaf(w, vprofile(g, vol + ((size_t)ix * g.ny + iy) * g.nz, C.mz, C.inv_mz, Va, Vb, inv_dv),
-                    part);
+// LONG: running sums of the volume's columns over z, from 0 again every 1 << lz slices
+// (from the volume's start they would carry the rounding of the column's total).
+__global__ void __launch_bounds__(256)
+sf3d_zsums(vg_dd3d_geom g, const float *__restrict__ vol, int lz, float *__restrict__ zs) {
+    const int lane = threadIdx.x & 31, per = (g.nz + 31) >> 5;
+    const size_t n = (size_t)g.nx * g.ny * per;
+    for (size_t w = ((size_t)blockIdx.x * 256 + threadIdx.x) >> 5; w < n; w += (size_t)gridDim.x * 8) {
+        const size_t col = w / per;
+        const int z = (int)(w - col * per) * 32 + lane;
+        float v = z < g.nz ? __ldg(vol + col * g.nz + z) : 0.f;
+        for (int o = 1; o < 1 << lz; o <<= 1) {
+            const float t = __shfl_up_sync(0xffffffffu, v, o);
+            if ((lane & ((1 << lz) - 1)) >= o) v += t;
+        }
+        if (z < g.nz) zs[col * g.nz + z] = v;
     }
-    return part;
 }
 
-template <int VEC, int M>
-__global__ void __launch_bounds__(32 * SFW, SF_FP_MINB)
+// LONG: a v cell from position tl to th, in slices from the c-th on: a part of its first
+// slice, those between, a part of its last.  f: the column, L: its running sums.
+__device__ __forceinline__ float long_cell(const float *f, const float *L, int nz, int lz, int c, float B, float tl,
+                                           float th) {
+    tl = fminf(fmaxf(tl, -1073741824.f), 1073741824.f);  // the rows below are int
+    th = fminf(fmaxf(th, -1073741824.f), 1073741824.f);
+    const float fl = floorf(tl), fh = floorf(th), w0 = fminf(B, (fl + 1.0f) - tl), w1 = fh > fl ? th - fh : 0.f;
+    const int r0 = c + (int)fl, r1 = c + (int)fh;
+    const int lo = max(r0 + 1, 0), hi = min(r1, nz);  // whole slices lo .. hi - 1
+    const bool whole = hi > lo;
+    const int b0 = lo >> lz, b1 = whole ? (hi - 1) >> lz : b0;
+    const float end = whole ? __ldg(L + hi - 1) : 0.f;
+    const float before = whole && (lo & ((1 << lz) - 1)) ? __ldg(L + lo - 1) : 0.f;
+    const float first = b0 < b1 ? __ldg(L + ((b0 + 1) << lz) - 1) : 0.f;
+    const float f0 = (unsigned)r0 < (unsigned)nz ? __ldg(f + r0) : 0.f;
+    const float f1 = w1 > 0.f && (unsigned)r1 < (unsigned)nz ? __ldg(f + r1) : 0.f;
+    float s = (first - before) + end;
+    for (int b = b0 + 1; b < b1; ++b) s += __ldg(L + ((b + 1) << lz) - 1);
+    s = fmaf(w0, f0, fmaf(w1, f1, s));
+    if (!(fabsf(s) < INFINITY)) {  // the running sums take infinities and NaN past their slice
+        s = 0.f;
+        for (int z = lo; z < hi; ++z) s += __ldg(f + z);
+        if ((unsigned)r0 < (unsigned)nz) s = fmaf(w0, __ldg(f + r0), s);
+        if (w1 > 0.f && (unsigned)r1 < (unsigned)nz) s = fmaf(w1, __ldg(f + r1), s);
+    }
+    return s;
+}
+
+template <int VEC, int M, bool LONG>
+__global__ void __launch_bounds__(32 * SFW, LONG ? SF_LONG_MINB : SF_FP_MINB)
 sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__restrict__ trig,
-               float *__restrict__ sino) {
+               float *__restrict__ sino, const float *__restrict__ zs, int lz) {
     constexpr int SZ = 32 * M, NW = M >= 2 ? 3 : 5;
     extern __shared__ float4 smem4[];
     const int ia = blockIdx.z, v0 = blockIdx.x * SZ;
@@ -246,6 +256,25 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
             grp[q / 2][m] = dup(0.f);
             acc[q * SZ + 32 * m] = 0.f;
         }
+    // a column's profile p at this lane's v cells to the 8 u cells
+    auto spread = [&](const float (&p)[M], bool odd, float4 wa, float4 wb) {
+        const float2 w2[UC / 2] = {make_float2(wa.x, wa.y), make_float2(wa.z, wa.w),
+                                   make_float2(wb.x, wb.y), make_float2(wb.z, wb.w)};
+        if (!__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+            for (int q = 0; q < UC / 2; ++q)
+#pragma unroll
+                for (int m = 0; m < M; ++m) grp[q][m] = pk_fma(w2[q], dup(p[m]), grp[q][m]);
+        } else {  // infinities and NaN only to the cells that the column covers
+#pragma unroll
+            for (int q = 0; q < UC / 2; ++q)
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    if (w2[q].x != 0.f) grp[q][m].x = fmaf(w2[q].x, p[m], grp[q][m].x);
+                    if (w2[q].y != 0.f) grp[q][m].y = fmaf(w2[q].y, p[m], grp[q][m].y);
+                }
+        }
+    };
     int ngrp = 0;
     for (int lb = 0; lb < no; lb += 32) {
         // columns of line lb + lane whose footprints can reach the cells: the map of
@@ -271,17 +300,16 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
             const int l = __ffs(lines) - 1, io = lb + l;
             lines &= lines - 1;
             const int ka = __shfl_sync(0xffffffffu, kA, l), ke = __shfl_sync(0xffffffffu, kE, l);
-            bool slow = ke - ka >= 32;
-            unsigned cols = 0;
-            if (!slow) {
+            bool some = false;
+            for (int kc = ka; kc <= ke; kc += 32) {  // 32 columns of the line at a time
                 // this lane's column
                 float w[UC];
                 float B = 1.f;
-                Win r = {};
+                Win wn = {};
                 int cidx = 0;
-                bool any = false, bad = false;
-                if (ka + lane <= ke) {
-                    const int k = ka + lane;
+                bool any = false;
+                if (kc + lane <= ke) {
+                    const int k = kc + lane;
                     const float cen = vox(g.d_pix, io, no), bx = vox(g.d_pix, k, nd);
                     const float x = xdrv ? bx : cen, y = xdrv ? cen : bx;
                     const SfCol C = sf_col(g, c, s, x, y);
@@ -296,36 +324,43 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
                             e = t;
                         }
                         B = kB * (g.DSO - fmaf(c, x, s * y));
-                        r = win_at<VEC>(B, B * vd, cf, ci, zn);
-                        if (r.start + r.rows <= 0 || r.start >= g.nz) any = false;
-                        bad = any && (B > NW - 1.0f || r.rows > BW - NW + 1);
+                        wn = win_at<VEC>(B, B * vd, cf, ci, zn);
+                        if (!LONG && (wn.start + wn.rows <= 0 || wn.start >= g.nz)) any = false;
                         cidx = xdrv ? k * g.ny + io : io * g.ny + k;
                     }
                 }
-                cols = __ballot_sync(0xffffffffu, any);
-                slow = __any_sync(0xffffffffu, bad);
+                unsigned cols = __ballot_sync(0xffffffffu, any);
+                if (!cols) continue;
+                some = true;
                 if (any) {
                     *reinterpret_cast<float4 *>(&W.w[lane][0]) = make_float4(w[0], w[1], w[2], w[3]);
                     *reinterpret_cast<float4 *>(&W.w[lane][4]) = make_float4(w[4], w[5], w[6], w[7]);
-                    W.rec[lane] = make_float4(B, r.y, __int_as_float(r.start), __int_as_float(cidx));
-                    W.mr[lane] = r.mid | r.rows << 12;
+                    W.rec[lane] = make_float4(B, wn.y, __int_as_float(LONG ? wn.start + wn.mid : wn.start),
+                                              __int_as_float(cidx));
+                    W.mr[lane] = wn.mid | wn.rows << 12;
                 }
                 __syncwarp();
-            }
-            if (slow) {
+                if (LONG) {
+                    for (; cols; cols &= cols - 1) {
+                        const int t = __ffs(cols) - 1;
+                        const float4 rc = W.rec[t];
+                        const int mid = max(min(__float_as_int(rc.z), 1 << 29), -(1 << 29));
+                        const size_t o = (size_t)__float_as_uint(rc.w) * g.nz;
+                        float p[M];
+                        bool odd = false;
 #pragma unroll
-                for (int q = 0; q < UC; ++q)
-#pragma unroll
-                    for (int m = 0; m < M; ++m) {
-                        const int iv = v0 + 32 * m + lane;
-                        if (q < nuT && iv < g.nv)
-                            (q & 1 ? grp[q / 2][m].y : grp[q / 2][m].x) +=
-                                sf_cell_line(g, vol, c, s, xdrv, nd, no, io, ka, ke, uedge(g, u0 + q),
-                                             uedge(g, u0 + q + 1), vedge(g, iv), vedge(g, iv + 1));
+                        for (int m = 0; m < M; ++m) {
+                            const float vm = (float)(min(32 * m + lane, zn - 1) - (zn >> 1));
+                            p[m] = long_cell(vol + o, zs + o, g.nz, lz, mid, rc.x, fmaf(rc.x, vm, rc.y),
+                                             fmaf(rc.x, vm + 1.0f, rc.y));
+                            odd |= !(fabsf(p[m]) < INFINITY);
+                        }
+                        spread(p, odd, *reinterpret_cast<const float4 *>(&W.w[t][0]),
+                               *reinterpret_cast<const float4 *>(&W.w[t][4]));
                     }
-            } else if (!cols) {
-                continue;
-            } else {
+                    __syncwarp();  // the table is reused
+                    continue;
+                }
                 int win = 0;
                 float2 r[2];
                 float4 rc;
@@ -403,26 +438,12 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
                         p[m] = a;
                         odd |= !(fabsf(a) < INFINITY);
                     }
-                    const float2 w2[UC / 2] = {make_float2(wa.x, wa.y), make_float2(wa.z, wa.w),
-                                               make_float2(wb.x, wb.y), make_float2(wb.z, wb.w)};
-                    if (!__any_sync(0xffffffffu, odd)) {
-#pragma unroll
-                        for (int q = 0; q < UC / 2; ++q)
-#pragma unroll
-                            for (int m = 0; m < M; ++m) grp[q][m] = pk_fma(w2[q], dup(p[m]), grp[q][m]);
-                    } else {  // infinities and NaN only to the cells that the column covers
-#pragma unroll
-                        for (int q = 0; q < UC / 2; ++q)
-#pragma unroll
-                            for (int m = 0; m < M; ++m) {
-                                if (w2[q].x != 0.f) grp[q][m].x = fmaf(w2[q].x, p[m], grp[q][m].x);
-                                if (w2[q].y != 0.f) grp[q][m].y = fmaf(w2[q].y, p[m], grp[q][m].y);
-                            }
-                    }
+                    spread(p, odd, wa, wb);
                     if (!cols) break;
                 }
                 __syncwarp();  // the table and the row buffers are reused
             }
+            if (!some) continue;
             if (++ngrp == 16) {
 #pragma unroll
                 for (int q = 0; q < UC; ++q)
@@ -449,14 +470,15 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
         }
 }
 
-template <int VEC, int M>
-int launch_fp(const vg_dd3d_geom *g, const float *vol, const double *trig, float *sino, cudaStream_t st) {
+template <int VEC, int M, bool LONG = false>
+int launch_fp(const vg_dd3d_geom *g, const float *vol, const double *trig, float *sino, cudaStream_t st,
+              const float *zs = nullptr, int lz = 0) {
     constexpr size_t smem = SFW * (sizeof(SfFpWarp) + UC * 32 * M * sizeof(float));
-    int s = cuda_status(cudaFuncSetAttribute(sf3d_fp_kernel<VEC, M>,
+    int s = cuda_status(cudaFuncSetAttribute(sf3d_fp_kernel<VEC, M, LONG>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "sf3d_fp");
     if (s) return s;
     dim3 grid(ceil_div(g->nv, 32 * M), ceil_div(g->nu, UC * SFW), g->na);
-    sf3d_fp_kernel<VEC, M><<<grid, 32 * SFW, smem, st>>>(*g, vol, trig, sino);
+    sf3d_fp_kernel<VEC, M, LONG><<<grid, 32 * SFW, smem, st>>>(*g, vol, trig, sino, zs, lz);
     return launch_status("sf3d_fp");
 }
 
@@ -862,7 +884,7 @@ size_t bp_ws_bytes(const vg_dd3d_geom *g) {
     return chunk_views(g) * (size_t)g->nu * g->nv * sizeof(float);
 }
 
-// kept from when the forward projection formed z sums of the volume's columns:
+// the forward projection's running sums over z (LONG); asked for in every geometry, as
 // callers size and check their workspace by it
 size_t fp_ws_bytes(const vg_dd3d_geom *g) {
     return (size_t)g->nx * g->ny * (g->nz + 1) * sizeof(float);
@@ -896,7 +918,18 @@ extern "C" int vg_sf3d_fp(const vg_dd3d_geom *g, const float *vol, const double 
         return vec ? launch_fp<4, 3>(g, vol, trig, sino, s) : launch_fp<1, 3>(g, vol, trig, sino, s);
     if (g->nv > 32 && 64.0 * bmax + 9.0 <= BW)
         return vec ? launch_fp<4, 2>(g, vol, trig, sino, s) : launch_fp<1, 2>(g, vol, trig, sino, s);
-    return vec ? launch_fp<4, 1>(g, vol, trig, sino, s) : launch_fp<1, 1>(g, vol, trig, sino, s);
+    if (32.0 * bmax + 9.0 <= BW)
+        return vec ? launch_fp<4, 1>(g, vol, trig, sino, s) : launch_fp<1, 1>(g, vol, trig, sino, s);
+    // v cells over more slices: running sums of about a cell's slices, so that a cell
+    // meets one end of them and carries their rounding
+    int lz = 2;
+    while (lz < 5 && (1 << lz) < bmax) ++lz;
+    float *zs = static_cast<float *>(workspace);
+    sf3d_zsums<<<1216, 256, 0, s>>>(*g, vol, lz, zs);
+    st = launch_status("sf3d_zsums");
+    if (st) return st;
+    return g->nv > 32 ? launch_fp<1, 2, true>(g, vol, trig, sino, s, zs, lz)
+                      : launch_fp<1, 1, true>(g, vol, trig, sino, s, zs, lz);
 }
 
 extern "C" int vg_sf3d_bp(const vg_dd3d_geom *g, const float *sino, const double *trig, float *vol,
