@@ -149,3 +149,28 @@ def test_sf_fp_long_cells_nonfinite_voxel(vg, value):
         x = torch.rand(shape, generator=torch.Generator().manual_seed(6)).cuda()
         x[at] = value
         assert torch.equal(~torch.isfinite(fp(x)), near)
+
+
+# shape, nu, nv, na, du, dv, d_pix, DSO, DSD: columns over more than 4 and more than 32 u
+# cells, slices over 4 to 30 v cells (pieces of 480), both, more slices than a warp's 32
+BP_WIDE = {
+    "u": ((11, 9, 33), 120, 50, 7, 0.2, 1.2, 1.0, 40.0, 70.0),
+    "u40": ((7, 6, 20), 500, 30, 5, 0.04, 1.2, 0.9, 30.0, 55.0),
+    "v": ((9, 10, 64), 26, 500, 7, 1.1, 0.3, 1.0, 40.0, 70.0),
+    "v30": ((6, 7, 40), 20, 2500, 5, 1.2, 0.06, 0.9, 40.0, 70.0),
+    "uv": ((8, 5, 37), 90, 300, 40, 0.25, 0.3, 1.0, 40.0, 70.0),
+    "beside": ((16, 17, 40), 30, 100, 20, 0.25, 0.3, 1.0, 40.0, 70.0),
+}
+
+
+@pytest.mark.parametrize("name", sorted(BP_WIDE))
+def test_sf_bp_wide_vs_oracle(vg, orc, name):
+    from vir_gb300.sys_mat import sp
+    shape, nu, nv, na, du, dv, d, DSO, DSD = BP_WIDE[name]
+    angs = np.linspace(0.03, 0.03 + 2 * np.pi, na, endpoint=False)
+    f = lambda v: float(np.float32(v))
+    kw = dict(du=f(du), dv=f(dv), su=f(0.3), sv=f(-0.4), d_pix=f(d))
+    y = np.random.default_rng(31).random((na, nu, nv)).astype(np.float32)
+    got = sp.sf_bp_cone_3d(y, angs, shape, DSO, DSD, **kw)
+    ref = orc.sf_bp_cone_3d(y, angs, shape, DSO, DSD, **kw)
+    assert np.abs(got - ref).max() <= 5e-5 * np.abs(ref).max()

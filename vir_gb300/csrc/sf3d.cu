@@ -510,7 +510,7 @@ __global__ void sf3d_weight(vg_dd3d_geom g, const float *__restrict__ sino, int 
 // Overlaps are in cell units, counted from the tile's middle.  Sums: 16
 // views in registers, then a compensated sum per voxel in shared memory.
 // Columns over more than 4 u cells, or whose slices reach more cells than the
-// buffer holds, take a per-voxel path.  With too few tiles to fill the GPU the
+// buffer holds, few here, take a per-voxel path.  With too few tiles to fill the GPU the
 // blocks of a cluster share a tile's views; sums meet in rank order.
 //
 // 256^3, 360 views of 512 x 384: 43.0 -> 16.6 ms (62 instructions per 32 voxels and
@@ -570,7 +570,7 @@ __device__ __noinline__ void sf_views_again(const vg_dd3d_geom &g, const float *
         }
 }
 
-constexpr int SF_BP_MINB = 3;
+constexpr int SF_BP_MINB = 3, SF_WIDE_MINB = 3;
 
 template <int VEC, int M>
 __global__ void __launch_bounds__(256, SF_BP_MINB)
@@ -852,6 +852,184 @@ int launch_bp(const vg_dd3d_geom *g, const float *qw, const double *trig, int a0
                        "sf3d_bp");
 }
 
+// Columns over any number of u cells, slices over any number of v cells (a warp: 8
+// columns of 32 slices, one view and column after the other).  The v cells that a
+// column's slices reach pass through the warp's buffer in pieces, the column's u cells
+// added up on the way; every lane then adds its slice's cells.  Up to 4 weights of a
+// column and its v map come from a table as in the column kernel; of wider ones the lanes
+// work out 32 weights at once.  Spare entries every 32 keep lanes 4, 8, 16 cells apart on
+// different banks.  Cells of no weight or overlap are left out.  Sums: 16 views, then
+// compensated.  128^3, 180 views, slices over 4 to 6 v cells: 8.1 -> 3.5 ms against the
+// column kernel's per-voxel path, columns over 7 to 12 u cells 27 -> 10.4 (4 blocks per SM,
+// with spills, 3.3 and 11.1).
+constexpr int WIDE_ROWS = 480;
+__device__ __forceinline__ int spare(int i) { return i + ((i >> 5) << 2); }
+struct SfWideWarp {
+    float T[WIDE_ROWS + WIDE_ROWS / 8];
+    float4 w[4][BT];    // F1 l_phi0 / dv of u cells j0 .. j0 + 3
+    float4 rec[4][BT];  // v cells per slice, Win's y and middle, j0 | count << 21
+    float grp[BT][32];
+    float2 kh[BT][32];  // (sum, compensation)
+};
+
+template <int VEC>
+__global__ void __launch_bounds__(256, SF_WIDE_MINB)
+sf3d_bp_wide_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__restrict__ trig, int a0, int cnt,
+                    int accumulate, float *__restrict__ vol) {
+    extern __shared__ float4 smem4[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    SfWideWarp &W = reinterpret_cast<SfWideWarp *>(smem4)[warp];
+    const int z0 = blockIdx.x * 32, iy = blockIdx.y * BT + warp, x0 = blockIdx.z * BT;
+    if (iy >= g.ny) return;  // no block barriers below
+    const int zn = min(32, g.nz - z0), nc = min(BT, g.nx - x0);
+    const float inv_du = 1.0f / g.du, U0 = uedge(g, 0);
+    const float zd = (float)(z0 + (zn >> 1)) - 0.5f * g.nz;  // the middle slice's edge
+    const float cv = 0.5f * g.nv - g.sv, ci = floorf(cv), cf = cv - ci;
+    for (int c = 0; c < BT; ++c) {
+        W.grp[c][lane] = 0.f;
+        W.kh[c][lane] = make_float2(0.f, 0.f);
+    }
+    for (int ib = 0; ib < cnt; ib += 4) {
+        {
+            const int sv = lane >> 3, c = lane & 7;
+            const float2 cs = view_cs(trig, a0 + min(ib + sv, cnt - 1));
+            float w[BKU] = {0.f, 0.f, 0.f, 0.f};
+            float B = 1.f;
+            Win wn = {};
+            int j0 = 0, n = 0;
+            if (c < nc) {
+                const SfCol C = sf_col(g, cs.x, cs.y, vox(g.d_pix, x0 + c, g.nx), vox(g.d_pix, iy, g.ny));
+                const int ja = max((int)floorf((C.t0 - U0) * inv_du), 0);
+                n = max(min((int)floorf((C.t3 - U0) * inv_du), g.nu - 1) - ja + 1, 0);
+                j0 = min(ja, g.nu - 1);
+                float e = trap_cum(uedge(g, j0), C);
+                const float f = inv_du * C.lphi;
+#pragma unroll
+                for (int t = 0; t < BKU; ++t) {
+                    const float h = trap_cum(uedge(g, j0 + t + 1), C);
+                    w[t] = t < n ? (h - e) * f : 0.f;
+                    e = h;
+                }
+                B = C.mz / g.dv;
+                wn = win_at<1>(B, B * zd, cf, ci, zn);
+            }
+            W.w[sv][c] = make_float4(w[0], w[1], w[2], w[3]);
+            W.rec[sv][c] = make_float4(B, wn.y, __int_as_float(max(min(wn.start + wn.mid, 1 << 29), -(1 << 29))),
+                                       __int_as_float(j0 | min(n, BKU + 1) << 21));  // nu < 2^21
+            __syncwarp();
+        }
+        const int nb = min(4, cnt - ib);
+        for (int sv = 0; sv < nb; ++sv) {
+            const float *q = qw + (size_t)(ib + sv) * g.nu * g.nv;
+            for (int c = 0; c < nc; ++c) {
+                const float4 rc = W.rec[sv][c];
+                const int bits = __float_as_int(rc.w), mid = __float_as_int(rc.z);
+                if (bits >> 21 == 0) continue;
+                const float B = rc.x;
+                const auto at = [&](int z) {  // slice z's first edge, in v cells from mid on
+                    return fminf(fmaxf(fmaf(B, (float)(z - (zn >> 1)), rc.y), -1073741824.f), 1073741824.f);
+                };
+                const int z = min(lane, zn - 1);
+                const float tl = at(z), th = at(z + 1), fl = floorf(tl), fh = floorf(th);
+                const int r0 = mid + (int)fl, r1 = mid + (int)fh;
+                const int la = max(__shfl_sync(0xffffffffu, r0, 0), 0) & ~(VEC - 1);
+                const int le = min(__shfl_sync(0xffffffffu, r1, zn - 1) + 1, g.nv);
+                const float w0 = fminf(B, (fl + 1.0f) - tl), w1 = fh > fl ? th - fh : 0.f;
+                float s = 0.f;
+                // the slices' sums of cells [l0, l0 + n) at T
+                auto add = [&](int l0, int n) {
+                    __syncwarp();
+                    const int e = min(r1 - l0, n);
+                    for (int i = max(r0 + 1 - l0, 0); i < e; ++i) s += W.T[spare(i)];
+                    if ((unsigned)(r0 - l0) < (unsigned)n) s = fmaf(w0, W.T[spare(r0 - l0)], s);
+                    if (w1 > 0.f && (unsigned)(r1 - l0) < (unsigned)n) s = fmaf(w1, W.T[spare(r1 - l0)], s);
+                    __syncwarp();
+                };
+                if (bits >> 21 <= BKU) {
+                    const float4 w = W.w[sv][c];
+                    const float *qj = q + (size_t)(bits & 0x1fffff) * g.nv;
+                    for (int l0 = la; l0 < le; l0 += WIDE_ROWS) {
+                        const int n = min(WIDE_ROWS, le - l0);
+                        for (int i = VEC * lane; i < n; i += 32 * VEC) {
+                            const float *p = qj + l0 + i;
+                            if (VEC == 4) {
+                                float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+                                auto mac = [&](float x, const float *p) {
+                                    const float4 f = __ldg(reinterpret_cast<const float4 *>(p));
+                                    o = make_float4(fmaf(x, f.x, o.x), fmaf(x, f.y, o.y), fmaf(x, f.z, o.z),
+                                                    fmaf(x, f.w, o.w));
+                                };
+                                if (w.x != 0.f) mac(w.x, p);
+                                if (w.y != 0.f) mac(w.y, p + g.nv);
+                                if (w.z != 0.f) mac(w.z, p + 2 * (size_t)g.nv);
+                                if (w.w != 0.f) mac(w.w, p + 3 * (size_t)g.nv);
+                                *reinterpret_cast<float4 *>(W.T + spare(i)) = o;
+                            } else {
+                                float o = w.x != 0.f ? w.x * __ldg(p) : 0.f;
+                                if (w.y != 0.f) o = fmaf(w.y, __ldg(p + g.nv), o);
+                                if (w.z != 0.f) o = fmaf(w.z, __ldg(p + 2 * (size_t)g.nv), o);
+                                if (w.w != 0.f) o = fmaf(w.w, __ldg(p + 3 * (size_t)g.nv), o);
+                                W.T[spare(i)] = o;
+                            }
+                        }
+                        add(l0, n);
+                    }
+                } else {
+                    const float2 cs = view_cs(trig, a0 + ib + sv);
+                    const SfCol C = sf_col(g, cs.x, cs.y, vox(g.d_pix, x0 + c, g.nx), vox(g.d_pix, iy, g.ny));
+                    const int jb = min((int)floorf((C.t3 - U0) * inv_du), g.nu - 1);
+                    for (int j0 = bits & 0x1fffff; j0 <= jb; j0 += 32) {
+                        const int nj = min(32, jb - j0 + 1);
+                        const float w =
+                            lane < nj ? uweight(C, uedge(g, j0 + lane), uedge(g, j0 + lane + 1), inv_du) : 0.f;
+                        for (int l0 = la; l0 < le; l0 += WIDE_ROWS) {
+                            const int n = min(WIDE_ROWS, le - l0);
+                            for (int i = 0; i < n; i += 32) {
+                                const float *p = q + (size_t)j0 * g.nv + (l0 + min(i + lane, n - 1));
+                                float o = 0.f;
+#pragma unroll 4
+                                for (int t = 0; t < nj; ++t, p += g.nv) {
+                                    const float wt = __shfl_sync(0xffffffffu, w, t);
+                                    if (wt != 0.f) o = fmaf(wt, __ldg(p), o);
+                                }
+                                W.T[spare(i + lane)] = o;
+                            }
+                            add(l0, n);
+                        }
+                    }
+                }
+                W.grp[c][lane] += s;
+            }
+        }
+        if ((ib & 15) == 12 || ib + 4 >= cnt)
+            for (int c = 0; c < nc; ++c) {
+                Kahan k;
+                k.s = W.kh[c][lane].x; k.c = W.kh[c][lane].y;
+                k.add(W.grp[c][lane]);
+                W.kh[c][lane] = make_float2(k.s, k.c);
+                W.grp[c][lane] = 0.f;
+            }
+        __syncwarp();  // the table is reused
+    }
+    if (lane < zn)
+        for (int c = 0; c < nc; ++c) {
+            float *o = vol + ((size_t)(x0 + c) * g.ny + iy) * g.nz + z0 + lane;
+            *o = accumulate ? *o + W.kh[c][lane].x : W.kh[c][lane].x;
+        }
+}
+
+template <int VEC>
+int launch_bp_wide(const vg_dd3d_geom *g, const float *qw, const double *trig, int a0, int cnt, float *vol,
+                   cudaStream_t st) {
+    constexpr size_t smem = 8 * sizeof(SfWideWarp);
+    int s = cuda_status(cudaFuncSetAttribute(sf3d_bp_wide_kernel<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem), "sf3d_bp_wide");
+    if (s) return s;
+    dim3 grid(ceil_div(g->nz, 32), ceil_div(g->ny, BT), ceil_div(g->nx, BT));
+    sf3d_bp_wide_kernel<VEC><<<grid, 256, smem, st>>>(*g, qw, trig, a0, cnt, (int)(a0 > 0), vol);
+    return launch_status("sf3d_bp_wide");
+}
+
 int check(const vg_dd3d_geom *g) {
     VG_REQUIRE(g, "sf3d: null geometry");
     VG_REQUIRE(g->nx > 0 && g->ny > 0 && g->nz > 0 && g->na > 0 && g->nu > 0 && g->nv > 0,
@@ -949,7 +1127,12 @@ extern "C" int vg_sf3d_bp(const vg_dd3d_geom *g, const float *sino, const double
     const double bmax = g->DSD / (g->DSO - fmin(r, 0.999 * g->DSO)) * g->d_pix / g->dv;
     const bool m2 = g->nz > 32 && 64.0 * bmax + 9.0 <= BW;
     const bool vec = g->nv % 4 == 0 && ((uintptr_t)qw & 15) == 0;
-    auto bp = m2 ? (vec ? launch_bp<4, 2> : launch_bp<1, 2>) : (vec ? launch_bp<4, 1> : launch_bp<1, 1>);
+    // the wide kernel where cells do not fit a row buffer, or columns reach 4.2 u cells, by
+    // the widest at the near side (128^3, 120 views: 1.7 against 1.9 ms at 4.0, 3.3 against
+    // 2.5 at 4.2)
+    const bool wide = (!m2 && 32.0 * bmax + 9.0 > BW) || 1.415 * bmax * g->dv / g->du > 4.2;
+    auto bp = wide ? (vec ? launch_bp_wide<4> : launch_bp_wide<1>)
+              : m2 ? (vec ? launch_bp<4, 2> : launch_bp<1, 2>) : (vec ? launch_bp<4, 1> : launch_bp<1, 1>);
     for (int a0 = 0; a0 < g->na; a0 += (int)nch) {
         const int cnt = (int)((size_t)(g->na - a0) < nch ? (size_t)(g->na - a0) : nch);
         sf3d_weight<<<1216, 256, 0, s>>>(*g, sino, a0, cnt, qw);
