@@ -96,7 +96,8 @@ __device__ __forceinline__ float lds_if(const float *p, float w) {
     float x = 0.f;
     asm volatile("{\n\t.reg .pred q;\n\tsetp.gt.f32 q, %2, 0f00000000;\n\t@q ld.shared.f32 %0, [%1];\n\t}"
                  : "+f"(x)
-                 : "r"((unsigned)__cvta_generic_to_shared(p)), "f"(w));
+                 : "r"((unsigned)__cvta_generic_to_shared(p)), "f"(w)
+                 : "memory");  // it reads what stores before it wrote
     return x;
 }
 
