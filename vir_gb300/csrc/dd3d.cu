@@ -593,14 +593,17 @@ dd3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const float4 *__re
             } else {
                 // the next 4 pixels of the cells over more than k0
                 auto more = [&](int k0) {
-                    if (!WIDE || !(wide4 >> (8 * sv) & 0xff)) return false;
-                    float w[4];
-                    int ks;
-                    const int n = columns(io, k0, w, ks);
-                    __syncwarp();
-                    put_column(W, sv, cs, w, ks, max(min(n - k0, 4), 0), ls == sv);
-                    __syncwarp();
-                    return __any_sync(0xffffffffu, n > k0) != 0;
+                    int n = 0;
+                    if constexpr (WIDE) {
+                        if (!(wide4 >> (8 * sv) & 0xff)) return false;
+                        float w[4];
+                        int ks;
+                        n = columns(io, k0, w, ks);
+                        __syncwarp();
+                        put_column(W, sv, cs, w, ks, max(min(n - k0, 4), 0), ls == sv);
+                        __syncwarp();
+                    }
+                    return WIDE && __any_sync(0xffffffffu, n > k0);
                 };
                 int k0 = 0;
                 if (WIDE && (long4 >> (8 * sv) & 1)) {
@@ -871,15 +874,18 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
                 } else {
                     // the next 4 detector columns of the voxels over more than k0
                     auto more = [&](int k0) {
-                        if (!WIDE || !(wide4 >> (8 * sv) & 0xff)) return false;
-                        const View3 v = view_f(vf, ia);
-                        float w[4];
-                        int js;
-                        const int n = columns(ia, v, k0, w, js);
-                        __syncwarp();
-                        put_column(W, sv, cs ^ (int)(v.pd < 0.f), w, js, max(min(n - k0, 4), 0), ls == sv);
-                        __syncwarp();
-                        return __any_sync(0xffffffffu, n > k0) != 0;
+                        int n = 0;
+                        if constexpr (WIDE) {
+                            if (!(wide4 >> (8 * sv) & 0xff)) return false;
+                            const View3 v = view_f(vf, ia);
+                            float w[4];
+                            int js;
+                            n = columns(ia, v, k0, w, js);
+                            __syncwarp();
+                            put_column(W, sv, cs ^ (int)(v.pd < 0.f), w, js, max(min(n - k0, 4), 0), ls == sv);
+                            __syncwarp();
+                        }
+                        return WIDE && __any_sync(0xffffffffu, n > k0);
                     };
                     int k0 = 0;
                     do {
