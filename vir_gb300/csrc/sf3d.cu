@@ -515,14 +515,16 @@ __global__ void sf3d_weight(vg_dd3d_geom g, const float *__restrict__ sino, int 
 //
 // 256^3, 360 views of 512 x 384: 43.0 -> 16.6 ms (62 instructions per 32 voxels and
 // view against 228, bound by issue and the latency of the loads; 2 blocks per SM
-// 18.1 ms).
+// 18.1 ms).  With 4-byte loads, or 32 slices, the 80 registers of 3 blocks spill: 2 there
+// (128 x 128 x 97, 180 views: 1.62 -> 1.52 ms).
 constexpr int BT = 8, BKU = 4;
 constexpr int BP_GROUP = 16;
 
 struct SfBpWarp {
     float T[2][2][BW];
     float4 w[4][BT];    // F1 l_phi0 / dv of u cells j0 .. j0 + 3
-    float4 rec[4][BT];  // v cells per slice, Win's y and start, j0 | count << 21 | Win's mid << 24
+    float4 rec[4][BT];  // v cells per slice, Win's y and start, j0 | count << 21
+    int mr[4][BT];      // Win's mid | rows << 12
 };
 
 // one voxel, one view, straight from the weighted sinogram (any geometry)
@@ -573,7 +575,7 @@ __device__ __noinline__ void sf_views_again(const vg_dd3d_geom &g, const float *
 constexpr int SF_BP_MINB = 3, SF_WIDE_MINB = 3;
 
 template <int VEC, int M>
-__global__ void __launch_bounds__(256, SF_BP_MINB)
+__global__ void __launch_bounds__(256, VEC == 1 || M == 1 ? 2 : SF_BP_MINB)
 sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__restrict__ trig, int a0,
                int cnt, int accumulate, float *__restrict__ vol) {
     constexpr int SZ = 32 * M, NW = M == 2 ? 3 : 5, NV = 4 / VEC;
@@ -587,8 +589,8 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
     const int iy = y0 + warp, zn = min(SZ, g.nz - z0);
     const float inv_du = 1.0f / g.du, U0 = uedge(g, 0);
     const float zd = (float)(z0 + (zn >> 1)) - 0.5f * g.nz;  // the middle slice's edge, exact
-    const float hi = (float)(zn - (zn >> 1));
     const float cv = 0.5f * g.nv - g.sv, ci = floorf(cv), cf = cv - ci;  // cell coordinate of v = 0
+    const float zl = (float)(lane - (zn >> 1));
     for (int c = warp; c < BT * BT; c += 8)
         for (int m = 0; m < M; ++m) kh[c * SZ + 32 * m + lane] = make_float2(0.f, 0.f);
     __syncthreads();
@@ -664,7 +666,8 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
             slow = __ballot_sync(0xffffffffu, n > BKU);
             live = __ballot_sync(0xffffffffu, n > 0);
             W.w[sv][c] = make_float4(w[0], w[1], w[2], w[3]);
-            W.rec[sv][c] = make_float4(B, r.y, __int_as_float(r.start), __int_as_float(j0 | n << 21 | r.mid << 24));
+            W.rec[sv][c] = make_float4(B, r.y, __int_as_float(r.start), __int_as_float(j0 | n << 21));
+            W.mr[sv][c] = r.mid | r.rows << 12;
             __syncwarp();
         }
         const int nb = min(4, va1 - ib);
@@ -703,9 +706,9 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
                 for (int h = 0; h < 2; ++h) {
                     const float4 w = W.w[sv][c0 + h], rc = W.rec[sv][c0 + h];
                     const int vs = __float_as_int(rc.z);
-                    const unsigned bits = __float_as_uint(rc.w), n = bits >> 21 & 7, mid = bits >> 24;
+                    const int bits = __float_as_int(rc.w), n = bits >> 21, mr = W.mr[sv][c0 + h], mid = mr & 0xfff;
                     const unsigned j = bits & 0x1fffff;  // nu < 2^21
-                    const int win = __float2int_rd(fmaf(rc.x, hi, rc.y)) + mid + NW;
+                    const int win = (mr >> 12) + NW - 1;
                     // this lane's cells, clamped to the window and the detector
                     int vo[NV];
                     unsigned in = 0;
@@ -757,14 +760,14 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
                     float over = 0.f;
 #pragma unroll
                     for (int m = 0; m < M; ++m) {
-                        const float zm = (float)(32 * m + lane - (zn >> 1));
+                        const float zm = zl + (float)(32 * m);
                         const float tl = fmaf(rc.x, zm, rc.y), th = fmaf(rc.x, zm + 1.0f, rc.y);
                         const float tf = floorf(tl);
                         wv[h][m][0] = fminf(th, tf + 1.0f) - tl;
 #pragma unroll
                         for (int t = 1; t < NW; ++t) wv[h][m][t] = __saturatef(th - (tf + (float)t));
                         if (32 * m + lane < zn) over = fmaxf(over, th - tf);
-                        qi[h][m] = min((int)tf + (int)mid, BW - NW);  // slices past the volume read anything
+                        qi[h][m] = min((int)tf + mid, BW - NW);  // slices past the volume read anything
                     }
                     two[h] = !__any_sync(0xffffffffu, over > 2.0f);
                     if (VEC == 4) {
