@@ -854,7 +854,8 @@ dd2d_fp_taps_kernel(vg_dd2d_geom g, const float *__restrict__ img, const float *
 // with the view loop unrolled by 4).  The tiles of a 512 x 512 image are 256
 // blocks, 1.7 per SM: in fan beam a cluster of blocks splits a tile's views until
 // an SM has four, which 64 registers and an unroll of 2 let it hold (0.204 ->
-// 0.184 ms; at 128 registers and an unroll of 4 a split tile takes 0.27 ms).
+// 0.184 ms; at 128 registers and an unroll of 4 a split tile takes 0.27 ms).  With
+// prep, 512 x 512, 720 views: split until two blocks 0.236 ms, four 0.205, eight 0.205.
 #ifndef VG_BP_TY
 #define VG_BP_TY 8
 #endif
@@ -1059,7 +1060,7 @@ int launch_bp_t(const vg_dd2d_geom *g, BpWork w, const double *trig, float *img,
     // block at least.  Parallel sums keep their order: SIRT divides by overlaps that
     // rounding alone makes at 0 and 90 degrees, and shows a last-bit change as 1e-3.
     int S = 1;
-    while (FAN && S < 4 && (long long)tx * ty * S < BP_FILL * 152 && g->na >= 32 * S) S *= 2;
+    while (FAN && S < 4 && (long long)tx * ty * S < BP_FILL * NSM && g->na >= 32 * S) S *= 2;
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3(ty * S, tx);
     c.blockDim = dim3(BP_TY, BP_TX);
@@ -1122,8 +1123,10 @@ int launch_fp_t(const vg_dd2d_geom *g, const float *img, const float *imgT, cons
 }
 
 // Whether the tap form is the one for the geometry: fan beam, bins of about 1.5
-// pixels at most at the isocentre (wider ones, whose pixels it would read one by
-// one, are the integral form's), the inverse map's pole so far off the
+// pixels at most at the isocentre (wider ones, of whose pixels it reads more and more
+// one by one, are left to the integral form: 512 x 512, 720 views, bins of 1.4
+// pixels 0.26 against 0.31 ms; of 1.8 it would still be 0.26 against 0.30, of 2.4 0.26
+// against 0.29), the inverse map's pole so far off the
 // detector that positions stay exact to the fraction where a bin meets the image
 // (|x| < 2^21): den >= 0.07 DSD, and no line nearer to the source of a diagonal view
 // than 0.18 of its distance: a bin is that much narrower on it, and the rounding of
@@ -1168,7 +1171,7 @@ int launch_taps(const vg_dd2d_geom *g, const float *img, const float *imgT, cons
     // whole views per block, or (never in mode 2) fewer bins until every SM has four blocks
     int cb = g->nu;
     if (mode != 2)
-        while (cb > 32 && (long long)g->na * ceil_div(g->nu, cb) < 4 * 152) cb = ((cb / 2 + 31) / 32) * 32;
+        while (cb > 32 && (long long)g->na * ceil_div(g->nu, cb) < 4 * NSM) cb = ((cb / 2 + 31) / 32) * 32;
     int LS = taps_split(cb);
     while (LS > 1 && taps_smem(g, cb, LS) > TAP_SMEM) LS /= 2;
     const size_t smem = taps_smem(g, cb, LS);

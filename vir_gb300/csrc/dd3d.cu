@@ -180,11 +180,11 @@ __device__ __noinline__ float fp_cell_line(const vg_dd3d_geom &g, const View3 &v
 // tabulated at once (lane = line or view x column) in the warp's own shared
 // memory: the warps of a block do not wait for each other.
 //
-// What bounds it: instruction issue (about 55 %) and the L1 data pipe (BP: 80 %,
-// from the v step, whose lanes are 1.15 rows apart and so hit a bank twice)
+// What bounds it: instruction issue (FP 56 %, BP 60 %) and the L1 data pipe (54 and
+// 79 %, from the v step, whose lanes are 1.15 rows apart and so hit a bank twice)
 // together.  Against the 3 x 3 gather through tables of all cells' overlaps, at
-// 256^3 voxels, 360 views of 512 x 384: FP 22.4 -> 13.3 ms, BP 17.3 -> 9.3 ms;
-// 512^3, 720 views of 1024 x 768: 634 -> 416 ms the pair.  Measured at 256^3 and
+// 256^3 voxels, 360 views of 512 x 384: FP 22.4 -> 13.1 ms, BP 17.3 -> 9.3 ms;
+// 512^3, 720 views of 1024 x 768: 634 -> 418 ms the pair.  Measured at 256^3 and
 // not kept: the detector window of a BP tile copied into shared memory by the
 // block, with 16-byte reads per column 15.6 ms, with 4 columns' rows side by
 // side 11.0 ms; that layout on global loads 12.6 ms.
@@ -937,10 +937,11 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
 }
 
 // Blocks of a cluster that share a tile: until every SM has about three blocks, 16
-// views per block at least.
+// views per block at least (360 views, until one, three and six blocks: 64^3 0.223,
+// 0.237 and 0.237 ms, 96^3 0.78, 0.85 and 0.72, 128^3 1.50, 1.50 and 1.25).
 int bp_split(const vg_dd3d_geom *g, long long tiles) {
     int S = 1;
-    while (S < 8 && tiles * S < 3 * 152 && g->na >= 32 * S) S *= 2;
+    while (S < 8 && tiles * S < 3 * NSM && g->na >= 32 * S) S *= 2;
     return S;
 }
 

@@ -37,7 +37,7 @@ __device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.
 // pass after pass, n = 1..3 at p entries each (fewer than N in all), and a block
 // filters several rows with it: read from W itself, 2^sh entries apart, they
 // took over half of the L1 cycles (at 69,120 rows of 512 with this and the spare
-// entries below 1.19 -> 0.97 ms, L1 89 -> 58 %; 512^3 FDK 109.1 -> 104.9 ms).
+// entries below 0.60 -> 0.49 ms, L1 89 -> 58 %; 512^3 FDK 109.1 -> 104.9 ms).
 __device__ __forceinline__ float2 tw(const float2 *t, int k, bool inv) {
     float2 w = t[k];
     if (inv) w.y = -w.y;
@@ -189,7 +189,7 @@ extern "C" int vg_filter_rows_fft(const float *in, int rows, int nu, int z, cons
     // block's table serves all of its rows; 16 waves, or registers bounded for
     // 5, 6 or 8 blocks, take the same time (105.2-106.0 ms FDK against 104.9)
     const size_t fit = (size_t)227 * 1024 / (smem + 1024);
-    const long long wave = 152LL * (fit < 1 ? 1 : fit < 6 ? fit : 6);
+    const long long wave = (long long)NSM * (fit < 1 ? 1 : fit < 6 ? fit : 6);
     filter_fft_kernel<<<(int)(rows < wave ? rows : wave), 256, smem, as_stream(stream)>>>(
         in, rows, nu, N, L, spectrum, reinterpret_cast<const float2 *>(twiddles), row_weight, out);
     return launch_status("filter_rows_fft");

@@ -134,7 +134,7 @@ __device__ __forceinline__ float unproj_idx(const vg_dd3d_geom &g, float c, floa
 // volume 9.1, 9.6 and 11.4; the slices through the row buffer 3.1, 1.9 and 2.0).  Sums:
 // 16 lines in registers, then a second running sum in shared memory.
 //
-// Bound by instruction issue (72 %, 213 per column and line for 8 x 96 cells).
+// Bound by instruction issue (66 %, 213 per column and line for 8 x 96 cells).
 // 256^3, 360 views of 512 x 384: 55.3 -> 21.6 ms against profiles of every column
 // in block-wide tables, one barrier per line (144 instructions per 32 cells and
 // line); the weights by branches per lane and the FMAs by cell 28 ms.  4 blocks
@@ -837,7 +837,7 @@ int launch_bp(const vg_dd3d_geom *g, const float *qw, const double *trig, int a0
     constexpr size_t smem = (size_t)BT * BT * 32 * M * sizeof(float2) + 8 * sizeof(SfBpWarp);
     const long long tiles = (long long)ceil_div(g->nz, 32 * M) * ceil_div(g->ny, BT) * ceil_div(g->nx, BT);
     int S = 1;
-    while (S < 8 && tiles * S < 3 * 152 && cnt >= 32 * S) S *= 2;
+    while (S < 8 && tiles * S < 3 * NSM && cnt >= 32 * S) S *= 2;
     int s = cuda_status(cudaFuncSetAttribute(sf3d_bp_kernel<VEC, M>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "sf3d_bp");
     if (s) return s;

@@ -108,6 +108,8 @@ __device__ __forceinline__ const char *ptr_at(const char *p, unsigned j, unsigne
     return q;
 }
 
+constexpr int NSM = 152;  // SMs of the GPU that grids are sized for
+
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace vg
