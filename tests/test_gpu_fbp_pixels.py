@@ -40,3 +40,29 @@ def test_fbp_pixels_vs_oracle(vg, orc, fan, shape, na, nu, su):
                _core.stream(qt.device))
     ref = orc.fbp2d_bp(q, angs, shape, fan=fan, DSO=DSO, DSD=DSD, du=du, su=f(su), d_pix=d)
     assert np.abs(img.cpu().numpy() - ref).max() <= 5e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("na", [20, 40, 200, 700])
+def test_infinite_bin_of_the_last_view(vg, na):
+    """An infinite bin of the last view is infinity, not NaN, where only the interpolation
+    towards it sees it, also where a tile's views are shared by several blocks (40 views and
+    more): the sums of parts keep it as the sum in one block does."""
+    import torch
+    from vir_gb300 import _core, _lib
+    nx, ny, nu, k = 40, 36, 64, 30
+    g = _lib.DD2DGeom(nx, ny, na, nu, 1.0, 0.0, 1.0, 60.0, 110.0, 1, 0)
+    trig = _core.trig_cache.get(np.linspace(0.1, 6.2, na), np.float32, torch.device("cuda", 0))
+
+    def bp(q):
+        out = torch.empty((nx, ny), device="cuda")
+        _lib.call("vg_fbp2d_bp", ctypes.byref(g), q.data_ptr(), trig.data_ptr(), out.data_ptr(), _core.stream())
+        return out
+
+    def bin_of(j, value):
+        q = torch.zeros((na, nu), device="cuda")
+        q[na - 1, j] = value
+        return bp(q)
+    # pixels between bins k - 1 and k: reached from bin k, and not from k + 1
+    want = (bin_of(k, 1.0) > 0) & ~(bin_of(k + 1, 1.0) > 0) & (bin_of(k - 1, 1.0) > 0)
+    assert bool(want.any())
+    assert bool(torch.isposinf(bin_of(k, float("inf")))[want].all())

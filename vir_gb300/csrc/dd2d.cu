@@ -1022,8 +1022,7 @@ __device__ __forceinline__ void bp_block(const vg_dd2d_geom &g, int tile_y, int 
                 Kahan a;
                 for (int r = 0; r < S; ++r) {
                     const float2 q = *cg::this_cluster().map_shared_rank(&sums[2 * dx + dy][tid], r);
-                    a.add(q.x);
-                    a.add(-q.y);
+                    a.merge(q);
                 }
                 acc[dx][dy] = a;
             }

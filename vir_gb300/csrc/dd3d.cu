@@ -919,8 +919,7 @@ dd3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ sino, const float4 *__r
             } else {
                 for (int r = 0; r < S; ++r) {
                     const float2 q = *cl.map_shared_rank(k, r);
-                    a.add(q.x);
-                    a.add(-q.y);
+                    a.merge(q);
                 }
             }
             const size_t o = ((size_t)ix * g.ny + iy) * g.nz + z0 + iz;

@@ -107,8 +107,7 @@ fbp2d_bp_kernel(vg_dd2d_geom g, const float *__restrict__ q, const double *__res
             for (int i = 0; i < PX; ++i)
                 for (int r = 1; r < S; ++r) {
                     const float2 a = *cl.map_shared_rank(&part[i][tid], r);
-                    acc[i].add(a.x);
-                    acc[i].add(-a.y);
+                    acc[i].merge(a);
                 }
         }
         cl.sync();  // no block leaves while its sums are read

@@ -820,8 +820,7 @@ sf3d_bp_kernel(vg_dd3d_geom g, const float *__restrict__ qw, const double *__res
             } else {
                 for (int r = 0; r < S; ++r) {
                     const float2 t = *cl.map_shared_rank(k, r);
-                    a.add(t.x);
-                    a.add(-t.y);
+                    a.merge(t);
                 }
             }
             float *o = vol + ((size_t)ix * g.ny + jy) * g.nz + z0 + iz;

@@ -45,6 +45,12 @@ struct Kahan {
         c = __fsub_rn(__fsub_rn(t, s), y);
         s = t;
     }
+    // another such sum (s, c); the compensation of an infinite one is NaN, which would
+    // make it NaN
+    __device__ __forceinline__ void merge(float2 q) {
+        add(q.x);
+        if (q.y == q.y) add(-q.y);
+    }
 };
 
 // FP64 helpers that keep every operation separately rounded, matching the
