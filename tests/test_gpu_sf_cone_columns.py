@@ -134,15 +134,16 @@ def test_sf_fp_wide_vs_oracle(vg, orc, name):
 
 
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
-def test_sf_fp_long_cells_nonfinite_voxel(vg, value):
-    """Where v cells take running sums, a voxel that is not finite makes exactly the cells
-    non-finite that a voxel of 1 in its place reaches."""
+@pytest.mark.parametrize("nz,nv,dv", [(160, 13, 13.3), (160, 300, 0.31), (61, 70, 1.13), (64, 30, 2.9)])
+def test_sf_fp_nonfinite_voxel_reaches_what_it_overlaps(vg, nz, nv, dv, value):
+    """A voxel that is not finite makes exactly the cells non-finite that a voxel of 1 in
+    its place reaches (running sums, 3 and 1 groups of v cells, 4- and 16-byte loads)."""
     import torch
     from vir_gb300.sys_mat import sp
-    shape, nu, nv, na = (14, 16, 160), 24, 13, 6
+    shape, nu, na = (14, 16, nz), 24, 6
     angs = np.linspace(0.1, 0.1 + 2 * np.pi, na, endpoint=False)
-    fp = lambda t: sp.sf_fp_cone_3d(t, angs, nu, nv, 60.0, 100.0, du=1.1, dv=13.3, su=0.31, sv=0.17, d_pix=0.7)
-    for at in ((3, 9, 80), (13, 0, 1), (7, 7, 158)):
+    fp = lambda t: sp.sf_fp_cone_3d(t, angs, nu, nv, 60.0, 100.0, du=1.1, dv=dv, su=0.31, sv=0.17, d_pix=0.7)
+    for at in ((3, 9, nz // 2), (13, 0, 1), (7, 7, nz - 2)):
         x = torch.zeros(shape, device="cuda")
         x[at] = 1.0
         near = fp(x) != 0

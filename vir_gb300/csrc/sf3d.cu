@@ -256,11 +256,12 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
             grp[q / 2][m] = dup(0.f);
             acc[q * SZ + 32 * m] = 0.f;
         }
-    // a column's profile p at this lane's v cells to the 8 u cells
+    // a column's profile p at this lane's v cells to the 8 u cells (odd: not finite in some
+    // lane)
     auto spread = [&](const float (&p)[M], bool odd, float4 wa, float4 wb) {
         const float2 w2[UC / 2] = {make_float2(wa.x, wa.y), make_float2(wa.z, wa.w),
                                    make_float2(wb.x, wb.y), make_float2(wb.z, wb.w)};
-        if (!__any_sync(0xffffffffu, odd)) {
+        if (!odd) {
 #pragma unroll
             for (int q = 0; q < UC / 2; ++q)
 #pragma unroll
@@ -355,7 +356,7 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
                                              fmaf(rc.x, vm + 1.0f, rc.y));
                             odd |= !(fabsf(p[m]) < INFINITY);
                         }
-                        spread(p, odd, *reinterpret_cast<const float4 *>(&W.w[t][0]),
+                        spread(p, __any_sync(0xffffffffu, odd), *reinterpret_cast<const float4 *>(&W.w[t][0]),
                                *reinterpret_cast<const float4 *>(&W.w[t][4]));
                     }
                     __syncwarp();  // the table is reused
@@ -437,6 +438,21 @@ sf3d_fp_kernel(vg_dd3d_geom g, const float *__restrict__ vol, const double *__re
                         }
                         p[m] = a;
                         odd |= !(fabsf(a) < INFINITY);
+                    }
+                    odd = __any_sync(0xffffffffu, odd);
+                    if (odd) {  // infinities and NaN only to the v cells that overlap them
+#pragma unroll
+                        for (int m = 0; m < M; ++m) {
+                            const float vm = (float)(32 * m + lane - (zn >> 1));
+                            const float tl = fmaf(cur.x, vm, cur.y), th = fmaf(cur.x, vm + 1.0f, cur.y);
+                            const float tf = floorf(tl);
+                            const float *q = T + min((int)tf + mid, BW - NW);
+                            p[m] = 0.f;
+                            for (int i = 0; i < NW; ++i) {
+                                const float wi = fminf(th, tf + (float)(i + 1)) - fmaxf(tl, tf + (float)i);
+                                if (wi > 0.f) p[m] = fmaf(wi, q[i], p[m]);
+                            }
+                        }
                     }
                     spread(p, odd, wa, wb);
                     if (!cols) break;
