@@ -137,3 +137,32 @@ def test_cone_sirt_wide_vs_unfused(vg, name):
         x = x + div(bp(div(y - fp(x), ws)), wi)
     near = wi > 1e-3 * wi.max()  # voxels beside the detector are divided by slivers
     assert (got - x).abs()[near].max() <= 1e-5 * x.abs()[near].max()
+
+
+@pytest.mark.parametrize("nz,nv,dv", [(64, 30, 2.9), (33, 20, 5.0), (30, 90, 1.1)])
+def test_cone_nonfinite_stays_within_a_row(vg, nz, nv, dv):
+    """A voxel or cell that is not finite reaches no output more than one row, or one
+    column, beside what it overlaps (1 and 2 groups of outputs, thin and thick slices)."""
+    import torch
+    from vir_gb300.sys_mat import dd
+    shape, nu, na = (14, 16, nz), 24, 6
+    angs = np.linspace(0.1, 0.1 + 2 * np.pi, na, endpoint=False)
+    kw = dict(du=1.1, dv=dv, su=0.31, sv=0.17, d_pix=0.7)
+    for call, size, rows in ((lambda t: dd.dd_fp_cone_3d(t, angs, nu, nv, 60.0, 100.0, **kw), shape, nz),
+                             (lambda t: dd.dd_bp_cone_3d(t, angs, shape, 60.0, 100.0, **kw), (na, nu, nv), nv)):
+        for z in (rows // 2,):  # away from the ends, where rows are read 4 at a time from the last
+            near = torch.zeros(call(torch.zeros(size, device="cuda")).shape, dtype=torch.bool, device="cuda")
+            for du in (-1, 0, 1):
+                for dz in (-1, 0, 1):
+                    x = torch.zeros(size, device="cuda")
+                    if size == shape:
+                        x[7, max(0, 9 + du) % 16, z + dz] = 1.0
+                        near |= call(x) != 0
+                        x.zero_()
+                        x[7 + du, 9, z + dz] = 1.0
+                    else:
+                        x[2, 12 + du, z + dz] = 1.0
+                    near |= call(x) != 0
+            x = torch.rand(size, generator=torch.Generator().manual_seed(6)).cuda()
+            x[(7, 9, z) if size == shape else (2, 12, z)] = float("inf")
+            assert not bool((~torch.isfinite(call(x)) & ~near).any())

@@ -341,7 +341,7 @@ struct Strip {
             a = fmaf(w[M - 1][1], t[1], a);
             if (!two) {
 #pragma unroll
-                for (int i = 2; i < NW; ++i) a = fmaf(w[M - 1][i], NW == 3 ? lds_if(t + i, w[M - 1][i]) : t[i], a);
+                for (int i = 2; i < NW; ++i) a = fmaf(w[M - 1][i], lds_if(t + i, w[M - 1][i]), a);
             }
             grp[M - 1] = a;
         }
