@@ -648,6 +648,12 @@ __device__ __forceinline__ float tap_lines(const float *__restrict__ px, const f
     return acc;
 }
 
+// tap_lines<0> out of line, for sums that are not finite
+__device__ __noinline__ float tap_lines_any(const float *px, const float4 *tab, TapBin b, int nd, int kofs, float zofs,
+                                            int io, int ie) {
+    return tap_lines<0>(px, tab, b, nd, kofs, zofs, io, ie);
+}
+
 // The same for lines (io, ie even) where all N pixels lie inside the line, two
 // lines per step in packed arithmetic.  FIRST: the share to first order in eps.
 template <bool FIRST, int N>
@@ -812,6 +818,9 @@ dd2d_fp_taps_kernel(vg_dd2d_geom g, const float *__restrict__ img, const float *
         a += tap_range<FIRST, 3>(base, tab, b, 2.f, nd, kofs, zofs, up ? c1 : c2, up ? c2 : c1);
         a += tap_range<FIRST, 4>(base, tab, b, 3.f, nd, kofs, zofs, up ? c2 : c3, up ? c3 : c2);
         a += tap_range<FIRST, 0>(base, tab, b, w, nd, kofs, zofs, up ? c3 : la, up ? lb : c3);
+        // infinities and NaN only to the bins that overlap them: the differences above take
+        // in a pixel of no weight too
+        if (!(fabsf(a) < INFINITY)) a = tap_lines_any(base, tab, b, nd, kofs, zofs, la, lb);
         if (e < nb) red[seg * cb + e] = a;
     }
     __syncthreads();
